@@ -76,10 +76,13 @@ def main():
             x = (torch.randn(M, K, device="cuda") * 0.5).bfloat16()
             row = {"shape": name, "K": K, "N": N, "M": M}
             if M <= Q.GEMV_MAX_M:
-                old = Q.GEMV_CHUNKED_MAX_M
-                Q.GEMV_CHUNKED_MAX_M = Q.GEMV_MAX_M      # force the GEMV for this batch size
+                old = Q.GEMV_CHUNKED_MAX_M, Q.ROWS_MAX_M
+                Q.GEMV_CHUNKED_MAX_M, Q.ROWS_MAX_M = Q.GEMV_MAX_M, 0      # force the GEMV for this batch size
                 row["gemv_us"] = round(graph_time_us(lambda i: Q.int4_matmul(x, qs[i])), 1)
-                Q.GEMV_CHUNKED_MAX_M = old
+                Q.GEMV_CHUNKED_MAX_M, Q.ROWS_MAX_M = old
+            if M <= Q.ROWS_MAX_M:
+                row["rows_us"] = round(graph_time_us(lambda i: Q.int4_matmul_rows(x, qs[i])), 1)
+                row["rows_frac_of_measured_hbm"] = round(packed_bytes / (row["rows_us"] * 1e-6) / (hbm * 1e9), 3)
             row["dequant_gemm_us"] = round(graph_time_us(lambda i: native.gemm(x, Q.int4_dequant(qs[i], x.dtype))), 1)
             y = Q.int4_matmul_fused(x, qs[0])
             if y is not None:

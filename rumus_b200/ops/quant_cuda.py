@@ -1,8 +1,9 @@
 """CUDA paths of the quantised matmuls (kernels: ``csrc/kernels/quant.cu``).
 
-INT4: small batches (decode) run the split-K GEMV that streams the packed weights once; larger
-``M`` expand the weight to a dense 16-bit matrix and run the tcgen05 GEMM; batches up to 128 rows
-can instead take the fused W4A16 tcgen05 kernel (opt-in, see ``w4a16_enabled``).
+INT4: 16-bit decode batches of up to 48 rows run the tensor-core kernel that feeds four-bit weights straight
+into registers (``csrc/kernels/int4_rows.cu``, groups that are multiples of 128); others of a few rows the
+split-K GEMV, of up to 48 rows the fused W4A16 tcgen05 kernel; larger ``M`` expand the weight to a dense
+16-bit matrix and run the tcgen05 GEMM.
 INT8 blocks: quantise / dequantise kernels; the matmul dequantises then uses the GEMM.
 """
 from __future__ import annotations
@@ -18,6 +19,7 @@ from ._lib import check, count_launch, ptr, stream_ptr
 P, I = c_void_p, c_int
 native.register_signature("rb_int4_gemv_splits", [I, I])
 native.register_signature("rb_int4_gemv", [I, I, P, P, P, P, P, P, P, I, I, I, I, I, P])
+native.register_signature("rb_int4_rows", [I, I, P, P, P, P, P, P, P, I, I, I, I, I, I, P])
 native.register_signature("rb_int4_dequant", [I, I, P, P, P, P, I, I, I, P])
 native.register_signature("rb_w4a16_slices", [I, I])
 native.register_signature("rb_w4a16_gemm", [I, I, P, c_longlong, P, P, P, P, P, P, P, I, I, I, I, I, P])
@@ -26,6 +28,8 @@ native.register_signature("rb_w8a16_gemm", [I, P, c_longlong, P, I, P, P, P, P, 
 native.register_signature("rb_q8_quantize", [I, P, P, I, I, I, P])
 native.register_signature("rb_q8_dequantize", [I, P, P, I, I, I, P])
 
+ROWS_MAX_M = 48            # rows of the register-fed tensor-core kernel; above, a dense copy is quicker (64 rows, the four
+                           # products of a 7B layer: 233 us by that kernel with eight groups of rows, 201 us)
 GEMV_MAX_M = 32            # rows one GEMV launch handles (accumulators in registers)
 GEMV_CHUNKED_MAX_M = 8     # batches up to this size use the GEMV; larger ones dequantise + tcgen05 GEMM
                            # (measured crossover on K 4096 x N 12288: GEMV 81 us at 8 rows, 118 us at 16;
@@ -115,14 +119,44 @@ def _gemv_scratch(device, numel: int) -> torch.Tensor:
     return buf
 
 
-def int4_matmul(x: torch.Tensor, qw, bias=None, out=None) -> torch.Tensor:
-    """x [M, K] @ dequant(qw) [K, N]; ``out`` (optional): contiguous ``[M, N]`` destination."""
+def int4_matmul_rows(x: torch.Tensor, qw, bias=None, out=None, residual=None, split: int = 0):
+    """The register-fed tensor-core kernel; returns ``None`` for shapes, types or alignments outside what it covers.
+    ``split``: CTAs that share K (0: chosen from the sizes)."""
+    M, K = x.shape
+    if M > ROWS_MAX_M or x.dtype not in (torch.bfloat16, torch.float16):
+        return None
+    x = x.contiguous()
+    y = out if out is not None else torch.empty((M, qw.n), dtype=x.dtype, device=x.device)
+    rc = native.lib().rb_int4_rows(native.dtype_code(x.dtype), native.dtype_code(qw.scales.dtype), ptr(x), ptr(qw.packed),
+                                   ptr(qw.scales), ptr(qw.zero_points), ptr(bias), ptr(residual), ptr(y), M, qw.n, K,
+                                   qw.padded_k, qw.group_size, split, stream_ptr())
+    if rc == 51:
+        return None
+    check(rc, "rb_int4_rows")
+    count_launch()
+    return y
+
+
+def int4_matmul(x: torch.Tensor, qw, bias=None, out=None, residual=None) -> torch.Tensor:
+    """x [M, K] @ dequant(qw) [K, N]; ``out`` (optional): contiguous ``[M, N]`` destination, ``residual`` (optional):
+    ``[M, N]`` that is added."""
     L = native.lib()
     M, K = x.shape
     assert K == qw.k
     x = x.contiguous()
     if out is not None:
         assert out.shape == (M, qw.n) and out.dtype == x.dtype and out.is_contiguous()
+    if residual is not None:
+        assert residual.shape == (M, qw.n) and residual.dtype == x.dtype
+        residual = residual.contiguous()
+    if bias is None or bias.dtype == x.dtype:
+        y = int4_matmul_rows(x, qw, bias, out, residual)
+        if y is not None:
+            return y
+    if residual is not None:
+        if M > W4A16_ROUTE_MAX_M:
+            return native.gemm(x, int4_dequant(qw, x.dtype), bias=bias, residual=residual, out=out)
+        return torch.add(residual, int4_matmul(x, qw, bias), out=out)
     if GEMV_CHUNKED_MAX_M < M <= W4A16_ROUTE_MAX_M and w4a16_enabled():
         y = int4_matmul_fused(x, qw, bias, out)
         if y is not None:

@@ -27,6 +27,7 @@ import torch.distributed as dist
 
 from ..models.registry import architecture_of
 from ..nn.quant import qmatmul_int4
+from ..ops.quant_cuda import int4_matmul
 from ..utils.metrics import trace_range
 from .batch import Portion, Segment, StepBatch
 from .cache import PagedKVCache
@@ -130,9 +131,8 @@ class Engine:
         partial result straight into a peer-visible buffer and ONE kernel does the flag round, the
         reduction over all ranks' partials and the residual add; NCCL mode: matmul, all-reduce, add."""
         if self.world == 1:
-            return residual + qmatmul_int4(h, qw)
+            return int4_matmul(h, qw, residual=residual) if h.is_cuda else residual + qmatmul_int4(h, qw)
         if self._ar and h.shape[0] * qw.n * h.element_size() <= self.ONESHOT_MAX_BYTES:
-            from ..ops.quant_cuda import int4_matmul
             from ..parallel import fused_ops
             T = h.shape[0]
             if self._capturing:
