@@ -8,17 +8,21 @@
 // Cache layout: k_cache / v_cache [num_blocks, block_size, Hkv, D] (token-major) or, in the `_hm`
 // entry points, [num_blocks, Hkv, block_size, D] (head-major); a sequence's logical token t lives in
 // physical block block_table[b][t / block_size] at offset t % block_size.
-#include "sm100_common.cuh"
+#include "warp_mma.cuh"
 
 namespace rb {
 
 constexpr int kPaWarps = 4;
+constexpr int kPaStages = 3;       // pairs of tokens of every 8-lane group in shared memory or on their way
 
 // grid (H, B, splits), 128 threads.  D = 128: eight lanes share one token (16 dims = two 16-byte
 // loads of K and of V per lane), so a warp works on four tokens at once and every 8-lane group
-// carries its own online-softmax state; two tokens per group are in flight per trip.  (One token
-// per warp with 8-byte loads left the kernel latency bound at about half the HBM rate.)
-// partial_o [B,H,splits,D] fp32, partial_ml [B,H,splits,2] (running max in log2 domain, sum).
+// carries its own online-softmax state.  Bound by the cache's way from HBM: a lane copies its pieces
+// of the next pairs of tokens (cp.async) into a ring that only the lane itself reads, so up to two pairs
+// of every group are in flight while one is computed, without registers for them or barriers.  (Plain loads,
+// used in the trip that asked for them: 225 us for 48 sequences of 1100 tokens, 32 heads, 865 MB.)
+// partial_o [B,H,splits,D] fp32, partial_ml [B,H,splits,2] (running max in log2 domain, sum); with one split
+// the result is written at once.
 template <typename T>
 __device__ __forceinline__ void pa_load16(const T* p, float* f) {
   const uint4 a = *reinterpret_cast<const uint4*>(p);
@@ -31,19 +35,37 @@ __device__ __forceinline__ void pa_load16(const T* p, float* f) {
     f[8 + j] = to_f32<T>(eb[j]);
   }
 }
+// the sixteen numbers of a lane's two pieces in the ring, 512 bytes (one warp) apart
+template <typename T>
+__device__ __forceinline__ void pa_ring16(const uint8_t* p, float* f) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const uint4 a = *reinterpret_cast<const uint4*>(p + h * 512);
+    const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 v = unpack2<T>(w[j]);
+      f[h * 8 + 2 * j] = v.x;
+      f[h * 8 + 2 * j + 1] = v.y;
+    }
+  }
+}
 
 // HM = head-major cache [num_blocks, Hkv, block_size, D]: one head's tokens of a block are
 // contiguous (block_size * 256 B), so the four tokens a warp reads per trip are one 1 KiB run
-// instead of four 256-byte pieces a whole token row (Hkv * 256 B) apart.
+// instead of four 256-byte pieces a whole token row (Hkv * 256 B) apart.  block_shift: log2 of the block
+// size, or -1 when it is no power of two.
 template <typename T, bool HM = false>
 __global__ void __launch_bounds__(kPaWarps * 32)
-    paged_decode_attn_kernel(const T* __restrict__ q, const T* __restrict__ k_cache,
+    paged_decode_attn_kernel(const T* __restrict__ q, long long ldq, const T* __restrict__ k_cache,
                              const T* __restrict__ v_cache, const int* __restrict__ block_tables,
                              const int* __restrict__ ctx_lens, float* __restrict__ partial_o,
-                             float* __restrict__ partial_ml, int H, int Hkv, int block_size,
-                             int max_blocks, int splits, float scale_log2) {
+                             float* __restrict__ partial_ml, T* __restrict__ out, int H, int Hkv, int block_size,
+                             int block_shift, int max_blocks, int splits, float scale_log2) {
   constexpr int D = 128;
   constexpr int G = kPaWarps * 4;   // token groups per CTA
+  constexpr int STAGE = 8 * 512;    // of a warp: two tokens of a group, K and V, two pieces each
+  __shared__ __align__(16) uint8_t ring_all[kPaWarps * kPaStages * STAGE];
   const int h = blockIdx.x, b = blockIdx.y, sp = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int grp = lane >> 3, sub = lane & 7;
@@ -52,44 +74,56 @@ __global__ void __launch_bounds__(kPaWarps * 32)
   const int ctx = ctx_lens[b];
   const int per = (ctx + splits - 1) / splits;
   const int t0 = sp * per, t1 = min(ctx, t0 + per);
+  const int* table = block_tables + (long long)b * max_blocks;
+  uint8_t* ring = ring_all + warp * kPaStages * STAGE + lane * 16;
+  auto fetch = [&](int i) {
+    const uint32_t dst = smem_u32(ring + (i % kPaStages) * STAGE);
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int t = t0 + (2 * i + u) * G + gid;
+      if (t < t1) {
+        const int bi = block_shift >= 0 ? t >> block_shift : t / block_size;
+        const int off = t - bi * block_size;
+        const long long blk = table[bi];
+        long long at;
+        if constexpr (HM) at = ((blk * Hkv + hkv) * block_size + off) * D + sub * 16;
+        else at = ((blk * block_size + off) * Hkv + hkv) * D + sub * 16;
+        copy16(dst + (u * 4) * 512, k_cache + at, true);
+        copy16(dst + (u * 4 + 1) * 512, k_cache + at + 8, true);
+        copy16(dst + (u * 4 + 2) * 512, v_cache + at, true);
+        copy16(dst + (u * 4 + 3) * 512, v_cache + at + 8, true);
+      }
+    }
+    copy_commit();
+  };
+  const int trips = t1 > t0 ? (t1 - t0 + 2 * G - 1) / (2 * G) : 0;
+#pragma unroll
+  for (int i = 0; i < kPaStages - 1; ++i) fetch(i);
   float qv[16];
-  pa_load16<T>(q + ((long long)b * H + h) * D + sub * 16, qv);
+  pa_load16<T>(q + (long long)b * ldq + h * D + sub * 16, qv);
 #pragma unroll
   for (int j = 0; j < 16; ++j) qv[j] *= scale_log2;
   float m = -INFINITY, l = 0.f, acc[16];
 #pragma unroll
   for (int j = 0; j < 16; ++j) acc[j] = 0.f;
-  const int* table = block_tables + (long long)b * max_blocks;
-  auto row_base = [&](int t) -> long long {
-    const int blk = table[t / block_size];
-    if constexpr (HM)
-      return (((long long)blk * Hkv + hkv) * block_size + (t % block_size)) * D + sub * 16;
-    else
-      return (((long long)blk * block_size + (t % block_size)) * Hkv + hkv) * D + sub * 16;
-  };
   // every lane runs every trip (the shuffles are warp wide); out-of-range tokens are skipped
-  for (int tb = t0; tb < t1; tb += 2 * G) {
-    const int ta = tb + gid, tc = tb + G + gid;
+  for (int i = 0; i < trips; ++i) {
+    copy_wait<kPaStages - 2>();
+    fetch(i + kPaStages - 1);
+    const uint8_t* st = ring + (i % kPaStages) * STAGE;
+    const int ta = t0 + 2 * i * G + gid, tc = ta + G;
     const bool va = ta < t1, vc = tc < t1;
-    float ka[16], vaa[16], kc[16], vcc[16];
-    if (va) {
-      const long long base = row_base(ta);
-      pa_load16<T>(k_cache + base, ka);
-      pa_load16<T>(v_cache + base, vaa);
-    }
-    if (vc) {
-      const long long base = row_base(tc);
-      pa_load16<T>(k_cache + base, kc);
-      pa_load16<T>(v_cache + base, vcc);
-    }
+    float x[16];
     float sa = 0.f, sc = 0.f;
     if (va) {
+      pa_ring16<T>(st, x);
 #pragma unroll
-      for (int j = 0; j < 16; ++j) sa = fmaf(qv[j], ka[j], sa);
+      for (int j = 0; j < 16; ++j) sa = fmaf(qv[j], x[j], sa);
     }
     if (vc) {
+      pa_ring16<T>(st + 4 * 512, x);
 #pragma unroll
-      for (int j = 0; j < 16; ++j) sc = fmaf(qv[j], kc[j], sc);
+      for (int j = 0; j < 16; ++j) sc = fmaf(qv[j], x[j], sc);
     }
 #pragma unroll
     for (int o = 1; o < 8; o <<= 1) {
@@ -102,17 +136,22 @@ __global__ void __launch_bounds__(kPaWarps * 32)
       const float pa = fast_exp2(sa - mn);
       const float pc = vc ? fast_exp2(sc - mn) : 0.f;
       l = l * corr + pa + pc;
+      pa_ring16<T>(st + 2 * 512, x);
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        float v = acc[j] * corr + pa * vaa[j];
-        if (vc) v = fmaf(pc, vcc[j], v);
-        acc[j] = v;
+      for (int j = 0; j < 16; ++j) acc[j] = fmaf(pa, x[j], acc[j] * corr);
+      if (vc) {
+        pa_ring16<T>(st + 6 * 512, x);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) acc[j] = fmaf(pc, x[j], acc[j]);
       }
       m = mn;
     }
   }
-  // merge the 16 token groups of this CTA
-  __shared__ float s_m[G], s_l[G], s_acc[G][D];
+  // merge the 16 token groups of this CTA (their sums take the ring's place)
+  copy_wait<0>();
+  __syncthreads();
+  float(*s_acc)[D] = reinterpret_cast<float(*)[D]>(ring_all);
+  float *s_m = reinterpret_cast<float*>(ring_all) + G * D, *s_l = s_m + G;
   if (sub == 0) { s_m[gid] = m; s_l[gid] = l; }
 #pragma unroll
   for (int j = 0; j < 16; ++j) s_acc[gid][sub * 16 + j] = acc[j];
@@ -130,8 +169,12 @@ __global__ void __launch_bounds__(kPaWarps * 32)
       o += s_acc[g][d] * f;
     }
     const long long pi = ((long long)b * H + h) * splits + sp;
-    partial_o[pi * D + d] = o;
-    if (d == 0) { partial_ml[pi * 2] = gm; partial_ml[pi * 2 + 1] = gl; }
+    if (splits == 1) {
+      out[pi * D + d] = from_f32<T>(gl > 0.f ? o / gl : 0.f);
+    } else {
+      partial_o[pi * D + d] = o;
+      if (d == 0) { partial_ml[pi * 2] = gm; partial_ml[pi * 2 + 1] = gl; }
+    }
   }
 }
 
@@ -234,39 +277,58 @@ __global__ void __launch_bounds__(256)
 
 extern "C" {
 
-int rb_paged_decode_splits(int max_ctx) {
-  int s = (max_ctx + 511) / 512;
+// CTAs that share the keys of one (row, head): parts of at most 512 tokens, shorter ones (down to 64 tokens) while the rows and
+// heads alone leave less than four CTAs to an SM.
+int rb_paged_decode_splits(int max_ctx, int rows_heads) {
+  const int fill = (4 * rbh::sm_count() + rows_heads - 1) / (rows_heads > 0 ? rows_heads : 1);
+  int s = fill < (max_ctx + 63) / 64 ? fill : (max_ctx + 63) / 64;
+  if (s < (max_ctx + 511) / 512) s = (max_ctx + 511) / 512;
   if (s > 16) s = 16;
   if (s < 1) s = 1;
   return s;
 }
 
-// q [B,H,128]; out [B,H,128]; scratch_o: B*H*splits*128 floats; scratch_ml: B*H*splits*2 floats
-int rb_paged_decode_attn(int dtype, const void* q, const void* k_cache, const void* v_cache,
+}
+
+namespace rb {
+template <typename T, bool HM>
+static int paged_decode(const void* q, long long ldq, const void* k_cache, const void* v_cache, const int* block_tables,
+                        const int* ctx_lens, void* out, float* scratch_o, float* scratch_ml, int B, int H, int Hkv,
+                        int block_size, int max_blocks, int splits, float scale, cudaStream_t st) {
+  int shift = -1;
+  if ((block_size & (block_size - 1)) == 0)
+    for (shift = 0; (1 << shift) < block_size; ++shift) {}
+  paged_decode_attn_kernel<T, HM><<<dim3(H, B, splits), kPaWarps * 32, 0, st>>>(
+      (const T*)q, ldq, (const T*)k_cache, (const T*)v_cache, block_tables, ctx_lens, scratch_o, scratch_ml, (T*)out, H, Hkv,
+      block_size, shift, max_blocks, splits, scale * 1.4426950408889634f);
+  if (splits > 1) paged_decode_reduce_kernel<T><<<B * H, 128, 0, st>>>(scratch_o, scratch_ml, (T*)out, splits);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : 3000 + (int)e;
+}
+}  // namespace rb
+
+extern "C" {
+
+// q: rows of H * 128, ldq apart (a multiple of 8); out [B,H,128]; scratch_o: B*H*splits*128 floats; scratch_ml: B*H*splits*2 floats
+// (neither is used with one split).  head_major: the cache is [num_blocks, Hkv, block_size, 128].
+int rb_paged_decode_attn(int dtype, int head_major, const void* q, long long ldq, const void* k_cache, const void* v_cache,
                          const int* block_tables, const int* ctx_lens, void* out, float* scratch_o,
                          float* scratch_ml, int B, int H, int Hkv, int head_dim, int block_size,
                          int max_blocks, int splits, float scale, void* stream) {
   using namespace rb;
   if (head_dim != 128) return 20;
   if (B <= 0) return 0;
+  if (ldq % 8) return 21;
   cudaStream_t st = (cudaStream_t)stream;
-  dim3 grid(H, B, splits);
-  const float sl2 = scale * 1.4426950408889634f;
-  if (dtype == rbh::DT_BF16) {
-    paged_decode_attn_kernel<__nv_bfloat16><<<grid, kPaWarps * 32, 0, st>>>(
-        (const __nv_bfloat16*)q, (const __nv_bfloat16*)k_cache, (const __nv_bfloat16*)v_cache,
-        block_tables, ctx_lens, scratch_o, scratch_ml, H, Hkv, block_size, max_blocks, splits, sl2);
-    paged_decode_reduce_kernel<__nv_bfloat16><<<B * H, 128, 0, st>>>(scratch_o, scratch_ml, (__nv_bfloat16*)out, splits);
-  } else if (dtype == rbh::DT_F16) {
-    paged_decode_attn_kernel<__half><<<grid, kPaWarps * 32, 0, st>>>(
-        (const __half*)q, (const __half*)k_cache, (const __half*)v_cache, block_tables, ctx_lens,
-        scratch_o, scratch_ml, H, Hkv, block_size, max_blocks, splits, sl2);
-    paged_decode_reduce_kernel<__half><<<B * H, 128, 0, st>>>(scratch_o, scratch_ml, (__half*)out, splits);
-  } else {
-    return 20;
-  }
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : 3000 + (int)e;
+#define RB_PA(T)                                                                                                        \
+  (head_major ? paged_decode<T, true>(q, ldq, k_cache, v_cache, block_tables, ctx_lens, out, scratch_o, scratch_ml, B, \
+                                      H, Hkv, block_size, max_blocks, splits, scale, st)                                \
+              : paged_decode<T, false>(q, ldq, k_cache, v_cache, block_tables, ctx_lens, out, scratch_o, scratch_ml, B, \
+                                       H, Hkv, block_size, max_blocks, splits, scale, st))
+  if (dtype == rbh::DT_BF16) return RB_PA(__nv_bfloat16);
+  if (dtype == rbh::DT_F16) return RB_PA(__half);
+#undef RB_PA
+  return 20;
 }
 
 int rb_kv_append(int dtype, const void* k_src, const void* v_src, long long src_stride,
@@ -288,34 +350,7 @@ int rb_kv_append(int dtype, const void* k_src, const void* v_src, long long src_
   return e == cudaSuccess ? 0 : 3000 + (int)e;
 }
 
-// Head-major variants (cache [num_blocks, Hkv, block_size, 128]); same arguments otherwise.
-int rb_paged_decode_attn_hm(int dtype, const void* q, const void* k_cache, const void* v_cache,
-                            const int* block_tables, const int* ctx_lens, void* out, float* scratch_o,
-                            float* scratch_ml, int B, int H, int Hkv, int head_dim, int block_size,
-                            int max_blocks, int splits, float scale, void* stream) {
-  using namespace rb;
-  if (head_dim != 128) return 20;
-  if (B <= 0) return 0;
-  cudaStream_t st = (cudaStream_t)stream;
-  dim3 grid(H, B, splits);
-  const float sl2 = scale * 1.4426950408889634f;
-  if (dtype == rbh::DT_BF16) {
-    paged_decode_attn_kernel<__nv_bfloat16, true><<<grid, kPaWarps * 32, 0, st>>>(
-        (const __nv_bfloat16*)q, (const __nv_bfloat16*)k_cache, (const __nv_bfloat16*)v_cache,
-        block_tables, ctx_lens, scratch_o, scratch_ml, H, Hkv, block_size, max_blocks, splits, sl2);
-    paged_decode_reduce_kernel<__nv_bfloat16><<<B * H, 128, 0, st>>>(scratch_o, scratch_ml, (__nv_bfloat16*)out, splits);
-  } else if (dtype == rbh::DT_F16) {
-    paged_decode_attn_kernel<__half, true><<<grid, kPaWarps * 32, 0, st>>>(
-        (const __half*)q, (const __half*)k_cache, (const __half*)v_cache, block_tables, ctx_lens,
-        scratch_o, scratch_ml, H, Hkv, block_size, max_blocks, splits, sl2);
-    paged_decode_reduce_kernel<__half><<<B * H, 128, 0, st>>>(scratch_o, scratch_ml, (__half*)out, splits);
-  } else {
-    return 20;
-  }
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : 3000 + (int)e;
-}
-
+// Head-major cache [num_blocks, Hkv, block_size, D].
 int rb_kv_append_hm(int dtype, const void* k_src, const void* v_src, long long src_stride,
                     const long long* slots, void* k_cache, void* v_cache, int tokens, int Hkv, int D,
                     int block_size, void* stream) {

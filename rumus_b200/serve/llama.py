@@ -7,7 +7,7 @@ or the fused W4A16 kernel, prefill the dequant + tcgen05 GEMM path.
 from __future__ import annotations
 
 import math
-from ctypes import c_float, c_int, c_void_p
+from ctypes import c_float, c_int, c_longlong, c_void_p
 from typing import List
 
 import torch
@@ -19,9 +19,8 @@ from .batch import StepBatch
 from .cache import PagedKVCache
 
 P, I, Fl = c_void_p, c_int, c_float
-native.register_signature("rb_paged_decode_splits", [I])
-native.register_signature("rb_paged_decode_attn", [I, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, Fl, P])
-native.register_signature("rb_paged_decode_attn_hm", [I, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, Fl, P])
+native.register_signature("rb_paged_decode_splits", [I, I])
+native.register_signature("rb_paged_decode_attn", [I, I, P, c_longlong, P, P, P, P, P, P, P, I, I, I, I, I, I, I, Fl, P])
 
 
 def paged_decode_attention(q, k_cache, v_cache, block_tables, ctx_lens, scale: float, max_ctx: int,
@@ -32,16 +31,19 @@ def paged_decode_attention(q, k_cache, v_cache, block_tables, ctx_lens, scale: f
     bs = k_cache.shape[2] if head_major else k_cache.shape[1]
     if q.is_cuda:
         L = native.lib()
-        splits = L.rb_paged_decode_splits(int(max_ctx))
-        so = torch.empty((B, H, splits, D), dtype=torch.float32, device=q.device)
-        sml = torch.empty((B, H, splits, 2), dtype=torch.float32, device=q.device)
-        out = torch.empty_like(q)
-        fn = L.rb_paged_decode_attn_hm if head_major else L.rb_paged_decode_attn
-        check(fn(native.dtype_code(q.dtype), ptr(q), ptr(k_cache), ptr(v_cache),
-                 ptr(block_tables), ptr(ctx_lens), ptr(out), ptr(so), ptr(sml), B, H,
-                 Hkv, D, bs, block_tables.shape[1], splits,
-                 float(scale), stream_ptr()), "rb_paged_decode_attn")
-        count_launch(2)
+        if q.stride(2) != 1 or q.stride(1) != D or q.stride(0) % 8 or q.data_ptr() % 16:
+            q = q.contiguous()
+        splits = L.rb_paged_decode_splits(int(max_ctx), B * H)
+        so = sml = None
+        if splits > 1:
+            so = torch.empty((B, H, splits, D), dtype=torch.float32, device=q.device)
+            sml = torch.empty((B, H, splits, 2), dtype=torch.float32, device=q.device)
+        out = torch.empty((B, H, D), dtype=q.dtype, device=q.device)
+        check(L.rb_paged_decode_attn(native.dtype_code(q.dtype), int(head_major), ptr(q), q.stride(0), ptr(k_cache), ptr(v_cache),
+                                     ptr(block_tables), ptr(ctx_lens), ptr(out), ptr(so), ptr(sml), B, H,
+                                     Hkv, D, bs, block_tables.shape[1], splits,
+                                     float(scale), stream_ptr()), "rb_paged_decode_attn")
+        count_launch(2 if splits > 1 else 1)
         return out
     outs = []
     for b in range(B):
@@ -181,7 +183,7 @@ class Int4LlamaShard:
         prompts on the keys just computed, continuations on the prefix gathered from the cache."""
         outs = []
         if batch.n_rows:
-            outs.append(paged_decode_attention(q[:batch.n_rows].contiguous(), cache.k[li], cache.v[li], batch.tables,
+            outs.append(paged_decode_attention(q[:batch.n_rows], cache.k[li], cache.v[li], batch.tables,
                                                batch.ctx, scale, batch.max_ctx, head_major=cache.head_major))
         for i, s in enumerate(batch.segments):
             r = slice(s.row0, s.row0 + s.n)
