@@ -10,17 +10,17 @@
 //     (g, t) has the words of columns 4 g .. 4 g + 3 at k = 8 t .. 8 t + 7, which are the left operands of two 16 x 16 tiles of
 //     two products, when the activations take the same order of k: nibbles p and p + 4 come out of a word together, so a piece
 //     of eight is read as (0 4) (1 5) (2 6) (3 7);
-//   * the operand is q - 8, which is exact in 16 bits; the products of a group are summed in fp32 and scaled in fp32 after it:
-//     acc += scale (sum (q - 8) x - (zp - 8) sum x).  So only the result is rounded, as in a product with fp32 weights.
-//     sum x of each group and row comes from a product with ones.
+//   * up to eight rows: the operand is q - 8, which is exact in 16 bits; the products of a group are summed in fp32 and scaled in fp32
+//     after it: acc += scale (sum (q - 8) x - (zp - 8) sum x), with sum x of each row from a product with ones.  Only the result is
+//     rounded, as in a product with fp32 weights.  More rows: the operand is (q - 8) scale + (8 - zp) scale in 16 bits, the
+//     weights of w4a16_gemm.cu, and all of K goes into one sum;
 //   * K is split over the warps of a CTA and, where the columns alone leave SMs idle, over a cluster of up to eight CTAs that
 //     add their sums through distributed shared memory in a fixed order: no workspace, no second launch.
 //
-// The four products of a 7B layer (4096 x 12288, 4096 x 4096, 4096 x 22016, 11008 x 4096), microseconds in all, against the streaming GEMV (1, 8 rows) and the tcgen05
-// kernel that expands weights into shared memory (16 to 48 rows):  1 row 61 (101),  8 rows 65 (210),  16: 92 (180),  24: 105 (201),  32: 118 (217),
-// 48: 169 (252); the weights' way from HBM is 17.  With one row the SMs' integer pipes (seven operations a word) and the wait for the first words share the rest,
-// with 48 rows the instructions of the products.  The result's error against 64 bits is that of its own rounding, 1.7e-3 in
-// bfloat16; weights expanded to 16 bits gave 2.9e-3.
+// The four products of a 7B layer (4096 x 12288, 4096 x 4096, 4096 x 22016, 11008 x 4096), microseconds in all, against the streaming GEMV (1, 8 rows) and
+// the tcgen05 kernel that expands weights into shared memory (16 to 48 rows):  1 row 62 (102),  8 rows 65 (212),  16: 85 (181),  24: 94 (203),
+// 32: 104 (219),  48: 132 (254); the weights' way from HBM is 17.  With few rows the SMs' integer pipes (seven operations a
+// word) and the wait for the first words share the rest, with many the instructions of the products.
 //
 // Packed layout (rumus-vision/src/quant.rs:42-126): word (k/8)*N + n holds k..k+7 of column n, nibble k%8; scales and zero
 // points are [K/group, N].
@@ -47,12 +47,14 @@ template <typename T> struct I4Num;
 template <> struct I4Num<__nv_bfloat16> {
   using V = __nv_bfloat162;
   static constexpr uint32_t magic = 0x43004300u, ones = 0x3f803f80u;      // 128 + q is exact
-  static __device__ __forceinline__ V base() { return __float2bfloat162_rn(136.f); }
+  static __device__ __forceinline__ V splat(float v) { return __float2bfloat162_rn(v); }
+  static __device__ __forceinline__ V base() { return splat(136.f); }
 };
 template <> struct I4Num<__half> {
   using V = __half2;
   static constexpr uint32_t magic = 0x64006400u, ones = 0x3c003c00u;      // 1024 + q is exact
-  static __device__ __forceinline__ V base() { return __float2half2_rn(1032.f); }
+  static __device__ __forceinline__ V splat(float v) { return __float2half2_rn(v); }
+  static __device__ __forceinline__ V base() { return splat(1032.f); }
 };
 
 template <typename T>
@@ -119,8 +121,8 @@ template <int NT_> struct I4Cfg {
   static constexpr int WARPS = 8, THREADS = 32 * WARPS;
   static constexpr int WK = WARPS / WN;
   static constexpr int COLS = 32 * WN;
-  static constexpr int STAGES = 3;
-  static constexpr int CTAS = NT <= 4 ? 2 : 1;      // per SM: the registers of the sums
+  static constexpr int STAGES = NT <= 4 ? 3 : 2;    // two CTAs of 48 rows fit an SM with two
+  static constexpr int CTAS = 2;                    // per SM
 };
 // a warp's share of a stage: words, scales, zero points
 template <typename TS> constexpr int i4_words_bytes() { return 2048 + 32 * 8 * (int)sizeof(TS); }
@@ -151,7 +153,6 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) int4_rows_kernel(const I4
   const int wn = warp % C::WN, wk = warp / C::WN;
   const int x_bytes = p.M * 256;                      // of one step
   const int stage_bytes = 8 * WB + C::WK * x_bytes;
-  float* sums = reinterpret_cast<float*>(smem + C::STAGES * stage_bytes);        // [2][WK][ROWS] (not ALONE)
   const int n0 = blockIdx.x * C::COLS;
   const int col = n0 + wn * 32 + 4 * g;
   const bool live = col < p.N;
@@ -240,26 +241,23 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) int4_rows_kernel(const I4
     at = at == C::STAGES - 1 ? 0 : at + 1;
     const uint8_t* words = stage + warp * WB;
     const uint8_t* sx = stage + 8 * WB + wk * x_bytes;
-    float* sm = sums + (i & 1) * C::WK * ROWS;
     const int base = s0 + i * C::WK;
     const bool work = base + wk < s1;
     fetch();
-    if constexpr (!ALONE) {
-      for (int u = warp; u < C::WK * NT; u += C::WARPS) {
-        const int w = u / NT, n = u - w * NT;
-        if (base + w < s1) {
-          const float2 v = sum_of(stage + 8 * WB + w * x_bytes, i4_x_at(min(n * 8 + g, p.M - 1), t));
-          if (g == 0) *reinterpret_cast<float2*>(sm + w * ROWS + n * 8 + 2 * t) = v;
+    if (work) {
+      float sc[4], zp[4];
+      i4_load4<TS>(words + 2048 + lane * 4 * sizeof(TS), sc);
+      i4_load4<TS>(words + 2048 + (32 + lane) * 4 * sizeof(TS), zp);
+      using V = typename I4Num<T>::V;
+      V s2[4], o2[4];
+      if constexpr (!ALONE) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          s2[k] = I4Num<T>::splat(sc[k]);
+          o2[k] = I4Num<T>::splat((8.f - zp[k]) * sc[k]);
         }
       }
-    }
-    float part[2][NT][4];
-    float2 xs[NT];
-    if (work) {
-      if constexpr (ALONE) {
-#pragma unroll
-        for (int n = 0; n < NT; ++n) xs[n] = sum_of(sx, xoff[n]);
-      }
+      float part[2][4];
       uint4 w = *reinterpret_cast<const uint4*>(words + lane * 16);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -273,6 +271,15 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) int4_rows_kernel(const I4
         i4_expand<T>(w.y, v[1]);
         i4_expand<T>(w.z, v[2]);
         i4_expand<T>(w.w, v[3]);
+        if constexpr (!ALONE) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const V r = __hfma2(*reinterpret_cast<V*>(&v[k][q]), s2[k], o2[k]);
+              v[k][q] = *reinterpret_cast<const uint32_t*>(&r);
+            }
+        }
         w = next;
 #pragma unroll
         for (int n = 0; n < NT; ++n) {
@@ -280,46 +287,35 @@ __global__ void __launch_bounds__(C::THREADS, C::CTAS) int4_rows_kernel(const I4
           const uint32_t b2 = __byte_perm(b[n].y, b[n].w, 0x5410), b3 = __byte_perm(b[n].y, b[n].w, 0x7632);
 #pragma unroll
           for (int a = 0; a < 2; ++a) {
-            if (j == 0) i4_mma_first<T>(part[a][n], v[2 * a][0], v[2 * a + 1][0], v[2 * a][1], v[2 * a + 1][1], b0, b1);
-            else i4_mma<T>(part[a][n], v[2 * a][0], v[2 * a + 1][0], v[2 * a][1], v[2 * a + 1][1], b0, b1);
+            float(&c)[4] = ALONE ? part[a] : acc[a][n];
+            if (ALONE && j == 0) i4_mma_first<T>(c, v[2 * a][0], v[2 * a + 1][0], v[2 * a][1], v[2 * a + 1][1], b0, b1);
+            else i4_mma<T>(c, v[2 * a][0], v[2 * a + 1][0], v[2 * a][1], v[2 * a + 1][1], b0, b1);
           }
 #pragma unroll
-          for (int a = 0; a < 2; ++a) i4_mma<T>(part[a][n], v[2 * a][2], v[2 * a + 1][2], v[2 * a][3], v[2 * a + 1][3], b2, b3);
+          for (int a = 0; a < 2; ++a) i4_mma<T>(ALONE ? part[a] : acc[a][n], v[2 * a][2], v[2 * a + 1][2], v[2 * a][3], v[2 * a + 1][3], b2, b3);
         }
       }
-    }
-    if constexpr (!ALONE) __syncthreads();         // the sums of all; and no warp reads this stage's activations any more
-    if (work) {
-      float sc[4], zp[4];
-      i4_load4<TS>(words + 2048 + lane * 4 * sizeof(TS), sc);
-      i4_load4<TS>(words + 2048 + (32 + lane) * 4 * sizeof(TS), zp);
-      float odd = 0.f;             // x - x is zero for a finite number only
-#pragma unroll
-      for (int n = 0; n < NT; ++n) {
-        if constexpr (!ALONE) xs[n] = *reinterpret_cast<const float2*>(sm + wk * ROWS + n * 8 + 2 * t);
-        odd += (xs[n].x - xs[n].x) + (xs[n].y - xs[n].y);
-      }
-      if (__any_sync(0xffffffffu, !(odd == 0.f))) {
-#pragma unroll
-        for (int n = 0; n < NT; ++n)
+      if constexpr (ALONE) {
+        const float2 xs = sum_of(sx, xoff[0]);
+        // x - x is zero for a finite number only
+        if (__any_sync(0xffffffffu, !((xs.x - xs.x) + (xs.y - xs.y) == 0.f))) {
 #pragma unroll
           for (int a = 0; a < 2; ++a)
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-              const int w = 2 * a + (c >> 1);
-              acc[a][n][c] += i4_plain<T>(words + g * 64, sx, min(n * 8 + 2 * t + (c & 1), p.M - 1), w, sc[w], zp[w]);
+              const int k = 2 * a + (c >> 1);
+              acc[a][0][c] += i4_plain<T>(words + g * 64, sx, min(2 * t + (c & 1), p.M - 1), k, sc[k], zp[k]);
             }
-      } else {
-#pragma unroll
-        for (int n = 0; n < NT; ++n)
+        } else {
 #pragma unroll
           for (int a = 0; a < 2; ++a) {
             const float z0 = 8.f - zp[2 * a], z1 = 8.f - zp[2 * a + 1];
-            acc[a][n][0] = fmaf(sc[2 * a], fmaf(z0, xs[n].x, part[a][n][0]), acc[a][n][0]);
-            acc[a][n][1] = fmaf(sc[2 * a], fmaf(z0, xs[n].y, part[a][n][1]), acc[a][n][1]);
-            acc[a][n][2] = fmaf(sc[2 * a + 1], fmaf(z1, xs[n].x, part[a][n][2]), acc[a][n][2]);
-            acc[a][n][3] = fmaf(sc[2 * a + 1], fmaf(z1, xs[n].y, part[a][n][3]), acc[a][n][3]);
+            acc[a][0][0] = fmaf(sc[2 * a], fmaf(z0, xs.x, part[a][0]), acc[a][0][0]);
+            acc[a][0][1] = fmaf(sc[2 * a], fmaf(z0, xs.y, part[a][1]), acc[a][0][1]);
+            acc[a][0][2] = fmaf(sc[2 * a + 1], fmaf(z1, xs.x, part[a][2]), acc[a][0][2]);
+            acc[a][0][3] = fmaf(sc[2 * a + 1], fmaf(z1, xs.y, part[a][3]), acc[a][0][3]);
           }
+        }
       }
     }
   }
@@ -389,7 +385,7 @@ int launch_int4_rows(I4Params p, int split, cudaStream_t st) {
   constexpr int ROWS = C::NT * 8;
   const int tiles = (p.N + C::COLS - 1) / C::COLS;
   const int red = 8 * 32 * ROWS * 4;
-  const int smem = max(C::STAGES * (8 * i4_words_bytes<TS>() + C::WK * p.M * 256) + 2 * C::WK * ROWS * 4, red);
+  const int smem = max(C::STAGES * (8 * i4_words_bytes<TS>() + C::WK * p.M * 256), red);
   if (smem > 227 * 1024) return 51;
   const int ctas = (smem + 1024) * C::CTAS <= 228 * 1024 ? C::CTAS : 1;
   // An SM's rounds, one CTA's after the other's, and what starting and finishing a wave of CTAs takes (about three rounds).  Clusters

@@ -26,8 +26,9 @@ def test_int4_rows(M, K, N, split):
     ref = x.double() @ q.dequantize(torch.float32).double()
     y = Q.int4_matmul_rows(x, q, split=split)
     # the result is rounded once to the 8 bits of bfloat16, which moves each value by at most 2^-8 of it (half of the 2^-7
-    # between neighbours at 1); the fp32 sums' own error is below 1e-5
-    assert _rel(y, ref) < 2 ** -8
+    # between neighbours at 1); the fp32 sums' own error is below 1e-5.  Above eight rows the weights are rounded too: scale,
+    # offset and weight by at most 2^-8 each, independently from weight to weight
+    assert _rel(y, ref) < (2 ** -8 if M <= 8 else 2 ** -7)
     assert torch.equal(y, Q.int4_matmul_rows(x, q, split=split))
 
 
@@ -39,7 +40,7 @@ def test_int4_rows_types_bias_residual(dtype, scale_dtype, M, group):
     bias, res = torch.randn(300, device="cuda").to(dtype), torch.randn(M, 300, device="cuda").to(dtype)
     ref = x.double() @ q.dequantize(torch.float32).double() + bias.double() + res.double()
     y = Q.int4_matmul(x, q, bias, residual=res)
-    assert _rel(y, ref) < (2 ** -8 if dtype is torch.bfloat16 else 2 ** -11)
+    assert _rel(y, ref) < (2 ** -8 if dtype is torch.bfloat16 else 2 ** -11) * (1 if M <= 8 else 2)
     out = torch.empty_like(y)
     assert Q.int4_matmul(x, q, bias, out=out, residual=res) is out and torch.equal(out, y)
     # above the kernel's rows: the same sum by the dense product
