@@ -23,10 +23,12 @@ constexpr int kPaStages = 3;       // pairs of tokens of every 8-lane group in s
 // used in the trip that asked for them: 225 us for 48 sequences of 1100 tokens, 32 heads, 865 MB.)
 // partial_o [B,H,splits,D] fp32, partial_ml [B,H,splits,2] (running max in log2 domain, sum); with one split
 // the result is written at once.
+// A lane's sixteen numbers of a row are its pieces sub and sub + 8 of sixteen: eight lanes copy 128 bytes side by side (with pieces 2 sub and
+// 2 sub + 1 each copy asked for half of every 32-byte sector, and each sector came twice: 240 us instead).
 template <typename T>
 __device__ __forceinline__ void pa_load16(const T* p, float* f) {
   const uint4 a = *reinterpret_cast<const uint4*>(p);
-  const uint4 b = *reinterpret_cast<const uint4*>(p + 8);
+  const uint4 b = *reinterpret_cast<const uint4*>(p + 64);
   const T* ea = reinterpret_cast<const T*>(&a);
   const T* eb = reinterpret_cast<const T*>(&b);
 #pragma unroll
@@ -86,12 +88,12 @@ __global__ void __launch_bounds__(kPaWarps * 32)
         const int off = t - bi * block_size;
         const long long blk = table[bi];
         long long at;
-        if constexpr (HM) at = ((blk * Hkv + hkv) * block_size + off) * D + sub * 16;
-        else at = ((blk * block_size + off) * Hkv + hkv) * D + sub * 16;
+        if constexpr (HM) at = ((blk * Hkv + hkv) * block_size + off) * D + sub * 8;
+        else at = ((blk * block_size + off) * Hkv + hkv) * D + sub * 8;
         copy16(dst + (u * 4) * 512, k_cache + at, true);
-        copy16(dst + (u * 4 + 1) * 512, k_cache + at + 8, true);
+        copy16(dst + (u * 4 + 1) * 512, k_cache + at + 64, true);
         copy16(dst + (u * 4 + 2) * 512, v_cache + at, true);
-        copy16(dst + (u * 4 + 3) * 512, v_cache + at + 8, true);
+        copy16(dst + (u * 4 + 3) * 512, v_cache + at + 64, true);
       }
     }
     copy_commit();
@@ -100,7 +102,7 @@ __global__ void __launch_bounds__(kPaWarps * 32)
 #pragma unroll
   for (int i = 0; i < kPaStages - 1; ++i) fetch(i);
   float qv[16];
-  pa_load16<T>(q + (long long)b * ldq + h * D + sub * 16, qv);
+  pa_load16<T>(q + (long long)b * ldq + h * D + sub * 8, qv);
 #pragma unroll
   for (int j = 0; j < 16; ++j) qv[j] *= scale_log2;
   float m = -INFINITY, l = 0.f, acc[16];
@@ -154,7 +156,7 @@ __global__ void __launch_bounds__(kPaWarps * 32)
   float *s_m = reinterpret_cast<float*>(ring_all) + G * D, *s_l = s_m + G;
   if (sub == 0) { s_m[gid] = m; s_l[gid] = l; }
 #pragma unroll
-  for (int j = 0; j < 16; ++j) s_acc[gid][sub * 16 + j] = acc[j];
+  for (int j = 0; j < 16; ++j) s_acc[gid][(j >> 3) * 64 + sub * 8 + (j & 7)] = acc[j];
   __syncthreads();
   {
     const int d = threadIdx.x;   // 128 threads, one output dim each
