@@ -245,6 +245,66 @@ __global__ void kv_append_hm_kernel(const T* __restrict__ k_src, const T* __rest
   }
 }
 
+// Rotary embedding of the query and key heads of packed rows [q | k | v] (pairs (i, i + hd/2)) in place, and the rotated keys and the values into the
+// cache: one pass over the rows where two rotations and an append take three.  A CTA per token (gridDim.y of them
+// share its heads): the angles are computed once per pair, not once per pair and head, and heads move in 16-byte pieces.
+// 1555 tokens of 32 + 32 heads: 15 us; 21.5 us a rotation and 7.8 us an append before.
+template <typename T, bool HM>
+__global__ void __launch_bounds__(256)
+    rope_append_kernel(T* __restrict__ qkv, long long ld, const long long* __restrict__ pos_ids, const long long* __restrict__ slots,
+                       T* __restrict__ k_cache, T* __restrict__ v_cache, int H, int Hkv, int hd, int block_size, float theta) {
+  extern __shared__ float s_angle[];                 // [hd/2] cosines, [hd/2] sines
+  const int half = hd / 2;
+  const long long t = blockIdx.x;
+  const float posf = (float)pos_ids[t];
+  for (int p = threadIdx.x; p < half; p += blockDim.x) {
+    const float inv_freq = __powf(theta, -2.0f * (float)p / (float)hd);
+    float sn, cs;
+    sincosf(posf * inv_freq, &sn, &cs);
+    s_angle[p] = cs;
+    s_angle[half + p] = sn;
+  }
+  __syncthreads();
+  T* row = qkv + t * ld;
+  const long long slot = slots[t];
+  auto place = [&](int hkv) -> long long {
+    if constexpr (HM) return (((slot / block_size) * Hkv + hkv) * block_size + slot % block_size) * hd;
+    else return (slot * Hkv + hkv) * hd;
+  };
+  const int first = blockIdx.y * blockDim.x + threadIdx.x, step = gridDim.y * blockDim.x;
+  const int per = half / 8;
+  for (int i = first; i < (H + Hkv) * per; i += step) {
+    const int h = i / per, c = (i - h * per) * 8;
+    T* base = row + (long long)h * hd + c;
+    const uint4 lo = *reinterpret_cast<const uint4*>(base), hi = *reinterpret_cast<const uint4*>(base + half);
+    const uint32_t l[4] = {lo.x, lo.y, lo.z, lo.w}, u[4] = {hi.x, hi.y, hi.z, hi.w};
+    uint32_t a[4], b[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 x = unpack2<T>(l[j]), y = unpack2<T>(u[j]);
+      const float c0 = s_angle[c + 2 * j], c1 = s_angle[c + 2 * j + 1];
+      const float s0 = s_angle[half + c + 2 * j], s1 = s_angle[half + c + 2 * j + 1];
+      a[j] = pack2<T>(x.x * c0 - y.x * s0, x.y * c1 - y.y * s1);
+      b[j] = pack2<T>(y.x * c0 + x.x * s0, y.y * c1 + x.y * s1);
+    }
+    const uint4 na = make_uint4(a[0], a[1], a[2], a[3]), nb = make_uint4(b[0], b[1], b[2], b[3]);
+    *reinterpret_cast<uint4*>(base) = na;
+    *reinterpret_cast<uint4*>(base + half) = nb;
+    if (h >= H && slot >= 0) {
+      T* dst = k_cache + place(h - H) + c;
+      *reinterpret_cast<uint4*>(dst) = na;
+      *reinterpret_cast<uint4*>(dst + half) = nb;
+    }
+  }
+  if (slot < 0) return;
+  const T* v = row + (long long)(H + Hkv) * hd;
+  const int vper = hd / 8;
+  for (int i = first; i < Hkv * vper; i += step) {
+    const int h = i / vper, c = (i - h * vper) * 8;
+    *reinterpret_cast<uint4*>(v_cache + place(h) + c) = *reinterpret_cast<const uint4*>(v + (long long)h * hd + c);
+  }
+}
+
 // out_idx[r] = argmax_c x[r, c] (first maximum), out_val[r] = the maximum
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -368,6 +428,24 @@ int rb_kv_append_hm(int dtype, const void* k_src, const void* v_src, long long s
     kv_append_hm_kernel<__half><<<blocks, 256, 0, st>>>((const __half*)k_src, (const __half*)v_src, src_stride, slots, (__half*)k_cache, (__half*)v_cache, tokens, Hkv, D, block_size);
   else
     return 20;
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : 3000 + (int)e;
+}
+
+// qkv: rows [H heads | Hkv heads | Hkv heads] of hd numbers, ld apart; hd a multiple of 16, ld of 8.  slot < 0: not stored.
+int rb_rope_append(int dtype, int head_major, void* qkv, long long ld, const long long* pos_ids, const long long* slots, void* k_cache,
+                   void* v_cache, int tokens, int H, int Hkv, int hd, int block_size, float theta, void* stream) {
+  using namespace rb;
+  if (tokens <= 0) return 0;
+  if (hd % 16 != 0 || hd > 1024 || ld % 8 != 0 || (reinterpret_cast<uintptr_t>(qkv) & 15)) return 21;
+  cudaStream_t st = (cudaStream_t)stream;
+  const dim3 grid(tokens, tokens < rbh::sm_count() ? 4 : 1);
+#define RB_ROPE_APPEND(T, HM) \
+  rope_append_kernel<T, HM><<<grid, 256, hd * sizeof(float), st>>>((T*)qkv, ld, pos_ids, slots, (T*)k_cache, (T*)v_cache, H, Hkv, hd, block_size, theta)
+  if (dtype == rbh::DT_BF16) { if (head_major) RB_ROPE_APPEND(__nv_bfloat16, true); else RB_ROPE_APPEND(__nv_bfloat16, false); }
+  else if (dtype == rbh::DT_F16) { if (head_major) RB_ROPE_APPEND(__half, true); else RB_ROPE_APPEND(__half, false); }
+  else return 20;
+#undef RB_ROPE_APPEND
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 3000 + (int)e;
 }

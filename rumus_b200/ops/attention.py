@@ -30,12 +30,14 @@ def _tma_ok(t: torch.Tensor) -> bool:
             and all((t.stride(i) * t.element_size()) % 16 == 0 for i in range(3)))
 
 
-def fa_forward(q, k, v, causal: bool, scale: float):
+def fa_forward(q, k, v, causal: bool, scale: float, out=None):
+    """``out``: contiguous ``[B, Sq, H, D]`` tensor to write the heads into."""
     L = native.lib()
     B, Sq, H, D = q.shape
     _, Sk, Hkv, _ = k.shape
     q, k, v = (t if _tma_ok(t) else t.contiguous() for t in (q, k, v))
-    o = torch.empty((B, Sq, H, D), dtype=q.dtype, device=q.device)
+    o = out if out is not None else torch.empty((B, Sq, H, D), dtype=q.dtype, device=q.device)
+    assert o.is_contiguous() and o.shape == q.shape and o.dtype == q.dtype
     lse = torch.empty((B, H, Sq), dtype=torch.float32, device=q.device)
     qs, ks, vs = _strides3(q), _strides3(k), _strides3(v)
     rc = L.rb_flash_attn_fwd(native.dtype_code(q.dtype), D, ptr(q), ptr(k), ptr(v),

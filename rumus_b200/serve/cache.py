@@ -3,7 +3,7 @@ lives at offset ``t % block_size`` of block ``table[t // block_size]`` in every 
 sequence lives in slots beside them."""
 from __future__ import annotations
 
-from ctypes import c_int, c_longlong, c_void_p
+from ctypes import c_float, c_int, c_longlong, c_void_p
 from typing import Dict, List, Optional, Tuple
 
 import torch
@@ -14,6 +14,7 @@ from ..ops._lib import check, count_launch, ptr, stream_ptr
 P, LL, I = c_void_p, c_longlong, c_int
 native.register_signature("rb_kv_append", [I, P, P, LL, P, P, P, I, I, P])
 native.register_signature("rb_kv_append_hm", [I, P, P, LL, P, P, P, I, I, I, I, P])
+native.register_signature("rb_rope_append", [I, I, P, LL, P, P, P, P, I, I, I, I, I, c_float, P])
 
 
 class PagedKVCache:
@@ -49,6 +50,16 @@ class PagedKVCache:
         else:
             kc.view(-1, row)[slots] = k_src
             vc.view(-1, row)[slots] = v_src
+
+    def rope_append(self, layer: int, qkv: torch.Tensor, heads: int, positions: torch.Tensor, slots: torch.Tensor, theta: float) -> None:
+        """Rotates the query and key heads of packed rows ``qkv [T, (heads + 2 Hkv) D]`` in place and stores keys and values
+        (GPU, 16-bit)."""
+        kc, vc = self.k[layer], self.v[layer]
+        assert qkv.dtype == kc.dtype and qkv.stride(1) == 1 and qkv.shape[1] == (heads + 2 * self.hkv) * self.hd
+        check(native.lib().rb_rope_append(native.dtype_code(kc.dtype), int(self.head_major), ptr(qkv), qkv.stride(0), ptr(positions),
+                                          ptr(slots), ptr(kc), ptr(vc), qkv.shape[0], heads, self.hkv, self.hd, self.block_size,
+                                          float(theta), stream_ptr()), "rb_rope_append")
+        count_launch()
 
     def gather(self, layer: int, table: torch.Tensor, positions: torch.Tensor):
         """K and V ``[len(positions), Hkv, D]`` of logical token ``positions`` of the sequence whose

@@ -13,7 +13,7 @@ from typing import List
 import torch
 
 from ..nn.quant import QuantizedTensor, qmatmul_int4
-from ..ops import functional as F, native
+from ..ops import attention, functional as F, native
 from ..ops._lib import check, count_launch, ptr, stream_ptr
 from .batch import StepBatch
 from .cache import PagedKVCache
@@ -24,8 +24,9 @@ native.register_signature("rb_paged_decode_attn", [I, I, P, c_longlong, P, P, P,
 
 
 def paged_decode_attention(q, k_cache, v_cache, block_tables, ctx_lens, scale: float, max_ctx: int,
-                           head_major: bool = False):
-    """q [B, H, D]; returns [B, H, D].  ``head_major``: cache is [blocks, Hkv, block_size, D]."""
+                           head_major: bool = False, out=None):
+    """q [B, H, D]; returns [B, H, D].  ``head_major``: cache is [blocks, Hkv, block_size, D].  ``out`` (GPU): contiguous
+    tensor to write into."""
     B, H, D = q.shape
     Hkv = k_cache.shape[1] if head_major else k_cache.shape[2]
     bs = k_cache.shape[2] if head_major else k_cache.shape[1]
@@ -38,7 +39,9 @@ def paged_decode_attention(q, k_cache, v_cache, block_tables, ctx_lens, scale: f
         if splits > 1:
             so = torch.empty((B, H, splits, D), dtype=torch.float32, device=q.device)
             sml = torch.empty((B, H, splits, 2), dtype=torch.float32, device=q.device)
-        out = torch.empty((B, H, D), dtype=q.dtype, device=q.device)
+        if out is None:
+            out = torch.empty((B, H, D), dtype=q.dtype, device=q.device)
+        assert out.is_contiguous() and out.shape == q.shape and out.dtype == q.dtype
         check(L.rb_paged_decode_attn(native.dtype_code(q.dtype), int(head_major), ptr(q), q.stride(0), ptr(k_cache), ptr(v_cache),
                                      ptr(block_tables), ptr(ctx_lens), ptr(out), ptr(so), ptr(sml), B, H,
                                      Hkv, D, bs, block_tables.shape[1], splits,
@@ -142,7 +145,9 @@ class Int4LlamaShard:
         self.ln_f = torch.ones(m.d_model, dtype=cfg.dtype, device=device)
         vloc = m.vocab_size // world
         self.vocab_local = vloc
-        self.head = rnd(m.d_model, m.vocab_size)[:, r * vloc:(r + 1) * vloc].contiguous().to(cfg.dtype).to(device)
+        # rows of K side by side: the product of a few rows (gemm_rows.cu) reads the weight that way; one row of 32000 x 4096 takes
+        # 48 us, 67 with rows of the vocabulary side by side
+        self.head = rnd(m.d_model, m.vocab_size)[:, r * vloc:(r + 1) * vloc].to(cfg.dtype).to(device).t().contiguous().t()
 
     # ------------------------------------------------------------------ what the engine calls
     tensor_parallel = True
@@ -162,17 +167,21 @@ class Int4LlamaShard:
         scale = 1.0 / math.sqrt(hd)
         x = F.embedding(batch.tokens, self.emb)
         T = x.shape[0]
+        fused = x.is_cuda and x.dtype in (torch.bfloat16, torch.float16) and hd % 16 == 0
         for li, L in enumerate(self.layers):
             h = F.rms_norm(x, L.ln1, eps)
             qkv = qmatmul_int4(h, L.qkv)
             q = qkv[:, : H * hd]
             k = qkv[:, H * hd: (H + Hkv) * hd]
             v = qkv[:, (H + Hkv) * hd:]
-            _rope(q, batch.positions, H, hd, m.rope_theta)
-            _rope(k, batch.positions, Hkv, hd, m.rope_theta)
-            cache.append(li, k, v, batch.slots)
+            if fused:
+                cache.rope_append(li, qkv, H, batch.positions, batch.slots, m.rope_theta)
+            else:
+                _rope(q, batch.positions, H, hd, m.rope_theta)
+                _rope(k, batch.positions, Hkv, hd, m.rope_theta)
+                cache.append(li, k, v, batch.slots)
             o = self._attend(li, q.reshape(T, H, hd), k.reshape(T, Hkv, hd), v.reshape(T, Hkv, hd), batch, cache, scale)
-            x = row_parallel(o.reshape(T, H * hd).contiguous(), L.out, x)
+            x = row_parallel(o.reshape(T, H * hd), L.out, x)
             h2 = F.rms_norm(x, L.ln2, eps)
             gu = qmatmul_int4(h2, L.gate_up)
             x = row_parallel(F.swiglu(gu), L.down, x)
@@ -181,17 +190,29 @@ class Int4LlamaShard:
     def _attend(self, li, q, k, v, batch: StepBatch, cache: PagedKVCache, scale: float):
         """Single tokens through the paged decode kernel; each prompt portion through FlashAttention, whole
         prompts on the keys just computed, continuations on the prefix gathered from the cache."""
-        outs = []
-        if batch.n_rows:
-            outs.append(paged_decode_attention(q[:batch.n_rows], cache.k[li], cache.v[li], batch.tables,
-                                               batch.ctx, scale, batch.max_ctx, head_major=cache.head_major))
+        if q.is_cuda:
+            T, H, D = q.shape
+            out = torch.empty((T, H, D), dtype=q.dtype, device=q.device)
+            if batch.n_rows:
+                paged_decode_attention(q[:batch.n_rows], cache.k[li], cache.v[li], batch.tables, batch.ctx, scale, batch.max_ctx,
+                                       head_major=cache.head_major, out=out[:batch.n_rows])
+        else:
+            outs = []
+            if batch.n_rows:
+                outs.append(paged_decode_attention(q[:batch.n_rows], cache.k[li], cache.v[li], batch.tables, batch.ctx, scale,
+                                                   batch.max_ctx, head_major=cache.head_major))
         for i, s in enumerate(batch.segments):
             r = slice(s.row0, s.row0 + s.n)
             kk, vv = k[r], v[r]
             if s.start:
                 kk, vv = cache.gather(li, batch.seg_tables[i].long(), torch.arange(s.start + s.n, device=q.device))
-            outs.append(F.flash_attention(q[r][None], kk[None], vv[None], True, scale)[0])
-        return outs[0] if len(outs) == 1 else torch.cat(outs)
+            if q.is_cuda and D in (64, 128) and q.dtype in (torch.bfloat16, torch.float16):
+                attention.fa_forward(q[r][None], kk[None], vv[None], True, scale, out=out[r][None])
+            elif q.is_cuda:
+                out[r] = F.flash_attention(q[r][None], kk[None], vv[None], True, scale)[0]
+            else:
+                outs.append(F.flash_attention(q[r][None], kk[None], vv[None], True, scale)[0])
+        return out if q.is_cuda else outs[0] if len(outs) == 1 else torch.cat(outs)
 
     def logits(self, hidden: torch.Tensor) -> torch.Tensor:
         return native.gemm(hidden.contiguous(), self.head) if hidden.is_cuda else hidden @ self.head
