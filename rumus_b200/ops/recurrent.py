@@ -103,7 +103,9 @@ def cut(portions, size: int, device) -> Chunks:
     for i, (row0, n) in enumerate(portions):
         items += [(row0 + at, min(size, n - at), i, 0) for at in range(0, n, size)]
         first.append(len(items))
-    both = torch.tensor([x for it in items for x in it] + first, dtype=torch.int32).to(device)
+    # from pinned memory: a copy from pageable memory would wait for what runs on the GPU
+    both = torch.tensor([x for it in items for x in it] + first, dtype=torch.int32,
+                        pin_memory=torch.device(device).type == "cuda").to(device, non_blocking=True)
     return Chunks(size, both[:4 * len(items)].view(-1, 4), both[4 * len(items):])
 
 

@@ -44,14 +44,24 @@ class StepBatch:
     # of the first token).  The first ``n_short`` stand in the single rows, the segments follow; no tokens: padding.
     seqs: Optional[torch.Tensor] = None      # int32 [n_short + len(segments), 4]
     n_short: int = 0
+    wanted: Optional[torch.Tensor] = None    # int64: rows whose logits are asked for, in the caller's order
 
     def to(self, device) -> "StepBatch":
-        """The same batch with its tensors on ``device`` (through pinned memory when that is a GPU)."""
-        gpu = torch.device(device).type == "cuda"
+        """The same batch with its tensors on ``device``: one copy of them all, which waits for nothing on a GPU."""
+        names = [n for n in ("tokens", "positions", "slots", "wanted", "tables", "ctx", "seg_tables", "seqs") if getattr(self, n) is not None]
+        parts = [getattr(self, n) for n in names]
+        sizes = [t.numel() * t.element_size() // 4 for t in parts]        # in int32
+        room = [-(-k // 64) * 64 for k in sizes]                           # every tensor starts on a 256-byte boundary
 
-        def move(t):
-            return t.pin_memory().to(device, non_blocking=True) if gpu else t.to(device)
+        def views(flat):
+            return [piece[:k].view(t.dtype).view(t.shape) for piece, k, t in zip(flat.split(room), sizes, parts)]
 
-        return replace(self, tokens=move(self.tokens), positions=move(self.positions), slots=move(self.slots),
-                       tables=move(self.tables), ctx=move(self.ctx), seg_tables=move(self.seg_tables),
-                       seqs=move(self.seqs))
+        host = torch.empty(sum(room), dtype=torch.int32, pin_memory=torch.device(device).type == "cuda")
+        for view, t in zip(views(host), parts):
+            view.copy_(t)
+        return replace(self, **dict(zip(names, views(host.to(device, non_blocking=True)))))
+
+
+def to_device(numbers, device, dtype=torch.int32) -> torch.Tensor:
+    """A list of numbers on ``device``, without waiting for what runs there (a copy from pageable memory would)."""
+    return torch.tensor(numbers, dtype=dtype, pin_memory=torch.device(device).type == "cuda").to(device, non_blocking=True)

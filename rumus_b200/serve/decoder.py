@@ -13,7 +13,7 @@ import torch
 from ..ops import native, recurrent
 from ..ops.latent import prefill_items
 from ..ops.stream import pad8, pad_heads, pad_to
-from .batch import StepBatch
+from .batch import StepBatch, to_device
 from .cache import HybridCache
 
 SHORT_PORTION = 8
@@ -30,7 +30,7 @@ class Step:
         self.batch, self.cache, self.tabs, self.items = batch, cache, tabs, None
         if batch.segments:
             segs = [(s.row0, s.n, i, s.start) for i, s in enumerate(batch.segments)]
-            self.items = torch.tensor(prefill_items(segs), dtype=torch.int32).to(cache.state.device)
+            self.items = to_device(prefill_items(segs), cache.state.device)
         self._chunks: dict = {}
 
     def chunks(self, size: int) -> recurrent.Chunks:

@@ -22,6 +22,7 @@ import time
 from dataclasses import dataclass, field
 from typing import Dict, List, Optional
 
+import numpy as np
 import torch
 import torch.distributed as dist
 
@@ -29,7 +30,7 @@ from ..models.registry import architecture_of
 from ..nn.quant import qmatmul_int4
 from ..ops.quant_cuda import int4_matmul
 from ..utils.metrics import trace_range
-from .batch import Portion, Segment, StepBatch
+from .batch import Portion, Segment, StepBatch, to_device
 from .cache import PagedKVCache
 from .llama import Int4LlamaShard, paged_decode_attention
 from .sampling import greedy_sample
@@ -163,21 +164,25 @@ class Engine:
         order = sorted(range(len(portions)), key=lambda i: limit is not None and lens[i] > limit)   # stable
         short = [i for i in order if limit is None or lens[i] <= limit]
         n_rows = sum(lens[i] for i in short)
-        tables = self.sched.block_tables([portions[i].rid for i in order], self.max_blocks)
-        n = torch.tensor([lens[i] for i in order])
-        start = torch.tensor([portions[i].start for i in order])
-        first = torch.cumsum(n, 0) - n
-        of = torch.repeat_interleave(torch.arange(len(order)), n)
-        pos = start[of] + torch.arange(of.shape[0]) - first[of]
-        slots = tables[of, pos // bs].long() * bs + pos % bs
+        rids = [portions[i].rid for i in order]
+        tables = self.sched.block_tables(rids, self.max_blocks)
+        n = np.array([lens[i] for i in order], dtype=np.int64)
+        start = np.array([portions[i].start for i in order], dtype=np.int64)
+        first = np.cumsum(n) - n
+        of = np.repeat(np.arange(len(order)), n)
+        pos = (start - first)[of] + np.arange(of.shape[0])
+        flat = tables.numpy()
+        slots = flat[of, pos // bs].astype(np.int64) * bs + pos % bs
         row0 = dict(zip(order, first.tolist()))
-        tokens = torch.tensor([t for i in order for t in portions[i].tokens], dtype=torch.int64)
+        tokens = np.array([t for i in order for t in portions[i].tokens], dtype=np.int64)
         segments = [Segment(portions[i].start, lens[i], row0[i]) for i in order[len(short):]]
-        ctx = (pos[:n_rows] + 1).to(torch.int32)
-        seqs = torch.stack([first.int(), n.int(), self.sched.places([portions[i].rid for i in order]), start.int()], 1)
-        batch = StepBatch(tokens, pos, slots, n_rows, tables[of[:n_rows]], ctx, int(ctx.max()) if n_rows else 0, segments,
-                          tables[len(short):], seqs, len(short))
-        return batch, [row0[i] + w for i, p in enumerate(portions) for w in p.want]
+        ctx = (pos[:n_rows] + 1).astype(np.int32)
+        seqs = np.stack([first, n, self.sched.places(rids).numpy(), start], 1).astype(np.int32)
+        rows = [row0[i] + w for i, p in enumerate(portions) for w in p.want]
+        host = torch.from_numpy
+        batch = StepBatch(host(tokens), host(pos), host(slots), n_rows, host(flat[of[:n_rows]]), host(ctx), int(ctx.max()) if n_rows else 0,
+                          segments, tables[len(short):], host(seqs), len(short), host(np.array(rows, dtype=np.int64)))
+        return batch, rows
 
     def _run(self, portions: List[Portion]) -> Optional[torch.Tensor]:
         """Computes one batch; returns the logits (this rank's part of the vocabulary) of the wanted tokens in
@@ -188,11 +193,13 @@ class Engine:
             if not batch.segments and self.cfg.cuda_graphs and self.device.type == "cuda":
                 hidden = self._decode_graph(batch)
             if hidden is None:
-                hidden = self.model.forward(batch.to(self.device), self.cache, self._row_parallel)
+                batch = batch.to(self.device)
+                hidden = self.model.forward(batch, self.cache, self._row_parallel)
         if not rows:
             return None
         if rows != list(range(hidden.shape[0])):
-            hidden = hidden.index_select(0, torch.tensor(rows, dtype=torch.int64, device=self.device))
+            wanted = batch.wanted if batch.wanted.device == hidden.device else to_device(rows, hidden.device, torch.int64)
+            hidden = hidden.index_select(0, wanted)
         return self.model.logits(hidden)
 
     def _argmax(self, logits: torch.Tensor) -> torch.Tensor:

@@ -22,7 +22,7 @@ from ..models.nufupel import MixtureConfig, NufupelConfig
 from ..ops import moe, native, stream, window
 from ..ops.latent import prefill_items
 from ..ops.stream import pad8, pad_heads, pad_to
-from .batch import StepBatch
+from .batch import StepBatch, to_device
 from .cache import PagedWindowCache
 
 SHORT_PORTION = 8
@@ -147,7 +147,7 @@ class NufupelServing:
         items = None
         if batch.segments:
             segs = [(s.row0, s.n, i, s.start) for i, s in enumerate(batch.segments)]
-            items = torch.tensor(prefill_items(segs), dtype=torch.int32).to(self.device)
+            items = to_device(prefill_items(segs), self.device)
         experts = None                   # what the previous layer's experts left, and which rows of it a token gains
         for li, L in enumerate(self.layers):
             a = L.cfg

@@ -19,7 +19,7 @@ import torch
 from ..models.zidalix import ZidalixConfig
 from ..ops import latent, native
 from ..ops.stream import pad8, pad_heads, pad_to
-from .batch import StepBatch
+from .batch import StepBatch, to_device
 from .cache import PagedLatentCache
 
 GLU_SLOPE, GLU_SHIFT = 1.702, 1.0
@@ -149,8 +149,8 @@ class ZidalixServing:
             segs.append((s.row0, s.n, off[-1], s.start))
             off.append(off[-1] + s.start + s.n)
         dev = self.device
-        return (torch.tensor(off, dtype=torch.int32).to(dev), off[-1],
-                torch.tensor(latent.prefill_items(segs), dtype=torch.int32).to(dev))
+        return (to_device(off, dev), off[-1],
+                to_device(latent.prefill_items(segs), dev))
 
     def _attend(self, L, proj: torch.Tensor, mix: torch.Tensor, batch: StepBatch, plan, pool: torch.Tensor) -> None:
         """Gated heads of every row into ``mix[:, :o_cols]``.  Single tokens attend in latent space; for prompt
