@@ -366,23 +366,40 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// Sums the slab partials of 32 channels with 8 slab slices per CTA; out2[0][c], out2[1][c] (smem)
-__device__ __forceinline__ void bn_fold_partials(const float* __restrict__ partials, int slabs,
-                                                 int C, int c, int slice, int cx, float& s,
-                                                 float& q, float (*ss)[33], float (*sq)[33]) {
+// Sums the slab partials of 8 channels (one 32-byte sector) with 32 slab slices per CTA, eight slabs of a slice in flight: what
+// counts is the chain of waits, not the bytes (up to 2048 slabs; with eight slices of 32 channels and one slab in flight 13 us).
+constexpr int kBnFoldCols = 8, kBnFoldSlices = 32;
+__device__ __forceinline__ void bn_fold_partials(const float* __restrict__ partials, int slabs, int C, int c, int slice, int cx,
+                                                 float& s, float& q) {
+  __shared__ float ss[kBnFoldSlices][kBnFoldCols + 1], sq[kBnFoldSlices][kBnFoldCols + 1];
   s = 0.f;
   q = 0.f;
-  if (c < C)
-    for (int i = slice; i < slabs; i += 8) {
+  if (c < C) {
+    int i = slice;
+    for (; i + 7 * kBnFoldSlices < slabs; i += 8 * kBnFoldSlices) {
+      float a[8], b[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        a[u] = partials[((long long)(i + u * kBnFoldSlices) * 2) * C + c];
+        b[u] = partials[((long long)(i + u * kBnFoldSlices) * 2 + 1) * C + c];
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        s += a[u];
+        q += b[u];
+      }
+    }
+    for (; i < slabs; i += kBnFoldSlices) {
       s += partials[((long long)i * 2) * C + c];
       q += partials[((long long)i * 2 + 1) * C + c];
     }
+  }
   ss[slice][cx] = s;
   sq[slice][cx] = q;
   __syncthreads();
   if (slice == 0) {
 #pragma unroll
-    for (int k = 1; k < 8; ++k) {
+    for (int k = 1; k < kBnFoldSlices; ++k) {
       s += ss[k][cx];
       q += sq[k][cx];
     }
@@ -394,11 +411,10 @@ __global__ void __launch_bounds__(256)
                                float eps, float momentum, float* __restrict__ mean,
                                float* __restrict__ rstd, float* __restrict__ running_mean,
                                float* __restrict__ running_var) {
-  __shared__ float ss[8][33], sq[8][33];
-  const int cx = threadIdx.x & 31, slice = threadIdx.x >> 5;
-  const int c = blockIdx.x * 32 + cx;
+  const int cx = threadIdx.x % kBnFoldCols, slice = threadIdx.x / kBnFoldCols;
+  const int c = blockIdx.x * kBnFoldCols + cx;
   float s, q;
-  bn_fold_partials(partials, slabs, C, c, slice, cx, s, q, ss, sq);
+  bn_fold_partials(partials, slabs, C, c, slice, cx, s, q);
   if (slice != 0 || c >= C) return;
   const float mu = s / (float)M;
   const float var = fmaxf(q / (float)M - mu * mu, 0.f);
@@ -415,11 +431,10 @@ __global__ void __launch_bounds__(256)
     bn_finalize_bwd_par_kernel(const float* __restrict__ partials, int slabs, int C,
                                float* __restrict__ sums, T* __restrict__ dgamma,
                                T* __restrict__ dbeta) {
-  __shared__ float ss[8][33], sq[8][33];
-  const int cx = threadIdx.x & 31, slice = threadIdx.x >> 5;
-  const int c = blockIdx.x * 32 + cx;
+  const int cx = threadIdx.x % kBnFoldCols, slice = threadIdx.x / kBnFoldCols;
+  const int c = blockIdx.x * kBnFoldCols + cx;
   float s, q;
-  bn_fold_partials(partials, slabs, C, c, slice, cx, s, q, ss, sq);
+  bn_fold_partials(partials, slabs, C, c, slice, cx, s, q);
   if (slice != 0 || c >= C) return;
   sums[c] = s;
   sums[C + c] = q;
@@ -641,50 +656,153 @@ __global__ void maxpool_nhwc_bwd_kernel(const T* __restrict__ dy, const signed c
     dx[i] = from_f32<T>(acc);
   }
 }
-// the same gather, eight channels (16 bytes of dy, 8 bytes of argmax codes) per thread
+// Eight channels (16 bytes) per thread.  KS: window size where the loads of a window are unrolled and all in flight (0: any size).
+// 256 images of 112 x 112 x 64, windows of 3: one channel a thread took 793 us (86 us is the way through HBM).
+template <typename T, int KS>
+__global__ void __launch_bounds__(256)
+    maxpool_nhwc_fwd_vec8_kernel(const T* __restrict__ x, T* __restrict__ y, signed char* __restrict__ idx, int B, int H, int W,
+                                 int C8, int k_any, int stride, int pad, int Ho, int Wo) {
+  const int K = KS ? KS : k_any;
+  const unsigned total = (unsigned)B * Ho * Wo * C8;
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    unsigned t = i / C8;
+    const int c8 = i - t * C8;
+    const int ow = t % Wo;
+    t /= Wo;
+    const int oh = t % Ho, b = t / Ho;
+    const uint4* base = reinterpret_cast<const uint4*>(x) + (long long)b * H * W * C8 + c8;
+    float best[8];
+    int bi[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) { best[j] = -INFINITY; bi[j] = -1; }
+    auto take = [&](const uint4& q, int code) {
+      const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 v = unpack2<T>(w[j]);
+        if (v.x > best[2 * j] || bi[2 * j] < 0) { best[2 * j] = v.x; bi[2 * j] = code; }
+        if (v.y > best[2 * j + 1] || bi[2 * j + 1] < 0) { best[2 * j + 1] = v.y; bi[2 * j + 1] = code; }
+      }
+    };
+    const int h0 = oh * stride - pad, w0 = ow * stride - pad;
+    if constexpr (KS > 0) {
+      uint4 q[KS * KS];
+      bool in[KS * KS];
+#pragma unroll
+      for (int k = 0; k < KS * KS; ++k) {
+        const int ih = h0 + k / KS, iw = w0 + k % KS;
+        in[k] = ih >= 0 && ih < H && iw >= 0 && iw < W;
+        if (in[k]) q[k] = base[(ih * W + iw) * C8];
+      }
+#pragma unroll
+      for (int k = 0; k < KS * KS; ++k)
+        if (in[k]) take(q[k], k);
+    } else {
+      for (int kh = 0; kh < K; ++kh)
+        for (int kw = 0; kw < K; ++kw) {
+          const int ih = h0 + kh, iw = w0 + kw;
+          if (ih >= 0 && ih < H && iw >= 0 && iw < W) take(base[(ih * W + iw) * C8], kh * K + kw);
+        }
+    }
+    uint32_t o[4], c[2] = {0, 0};
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if (bi[j] < 0) best[j] = 0.f;
+      c[j >> 2] |= (uint32_t)(bi[j] & 0xff) << (8 * (j & 3));
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o[j] = pack2<T>(best[2 * j], best[2 * j + 1]);
+    reinterpret_cast<uint4*>(y)[i] = make_uint4(o[0], o[1], o[2], o[3]);
+    reinterpret_cast<uint2*>(idx)[i] = make_uint2(c[0], c[1]);
+  }
+}
+// the same gather as above, eight channels (16 bytes of dy, 8 bytes of argmax codes) per thread; only the windows that hold the
+// pixel are visited, in the same order
 template <typename T>
-__global__ void maxpool_nhwc_bwd_vec8_kernel(const T* __restrict__ dy, const signed char* __restrict__ idx,
-                                             T* __restrict__ dx, int B, int H, int W, int C, int K,
-                                             int stride, int pad, int Ho, int Wo) {
-  const int C8 = C / 8;
-  const long long total = (long long)B * H * W * C8;
-  const long long gs = (long long)gridDim.x * blockDim.x;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gs) {
-    const int c8 = (int)(i % C8);
-    long long t = i / C8;
-    const int iw = (int)(t % W);
+__global__ void __launch_bounds__(256)
+    maxpool_nhwc_bwd_vec8_kernel(const T* __restrict__ dy, const signed char* __restrict__ idx,
+                                 T* __restrict__ dx, int B, int H, int W, int C8, int K,
+                                 int stride, int pad, int Ho, int Wo) {
+  const unsigned total = (unsigned)B * H * W * C8;
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    unsigned t = i / C8;
+    const int c8 = i - t * C8;
+    const int iw = t % W;
     t /= W;
-    const int ih = (int)(t % H);
-    const int b = (int)(t / H);
+    const int ih = t % H, b = t / H;
     float acc[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-    for (int kh = 0; kh < K; ++kh) {
-      const int nh = ih + pad - kh;
-      if (nh < 0 || nh % stride) continue;
-      const int oh = nh / stride;
-      if (oh >= Ho) continue;
-      for (int kw = 0; kw < K; ++kw) {
-        const int nw = iw + pad - kw;
-        if (nw < 0 || nw % stride) continue;
-        const int ow = nw / stride;
-        if (ow >= Wo) continue;
-        const long long o = (((long long)b * Ho + oh) * Wo + ow) * C + c8 * 8;
-        const uint2 codes = *reinterpret_cast<const uint2*>(idx + o);
-        const uint4 g = *reinterpret_cast<const uint4*>(dy + o);
-        const signed char* cd = reinterpret_cast<const signed char*>(&codes);
-        const T* ge = reinterpret_cast<const T*>(&g);
-        const int want = kh * K + kw;
+    const int h = ih + pad, w = iw + pad;
+    const int h_lo = h >= K ? (h - K) / stride + 1 : 0, h_hi = min(h / stride, Ho - 1);
+    const int w_lo = w >= K ? (w - K) / stride + 1 : 0, w_hi = min(w / stride, Wo - 1);
+    for (int oh = h_hi; oh >= h_lo; --oh)
+      for (int ow = w_hi; ow >= w_lo; --ow) {
+        const long long o = (((long long)b * Ho + oh) * Wo + ow) * C8 + c8;
+        const uint2 codes = reinterpret_cast<const uint2*>(idx)[o];
+        const uint4 g = reinterpret_cast<const uint4*>(dy)[o];
+        const uint32_t gw[4] = {g.x, g.y, g.z, g.w};
+        const uint32_t want = (uint32_t)((h - oh * stride) * K + w - ow * stride) & 0xff;
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-          if (cd[j] == want) acc[j] += to_f32<T>(ge[j]);
+        for (int j = 0; j < 8; ++j) {
+          const float2 v = unpack2<T>(gw[j >> 1]);
+          if ((((j < 4 ? codes.x : codes.y) >> (8 * (j & 3))) & 0xff) == want) acc[j] += (j & 1) ? v.y : v.x;
+        }
+      }
+    uint32_t o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o[j] = pack2<T>(acc[2 * j], acc[2 * j + 1]);
+    reinterpret_cast<uint4*>(dx)[i] = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+}
+// eight channels (16 bytes) per thread of the adaptive average pool below
+template <typename T, bool BWD>
+__global__ void __launch_bounds__(256)
+    adaptive_avgpool_nhwc_vec8_kernel(const T* __restrict__ src, T* __restrict__ dst, int B, int H, int W, int C8, int Ho, int Wo) {
+  const unsigned total = (unsigned)B * (BWD ? H * W : Ho * Wo) * C8;
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    unsigned t = i / C8;
+    const int c8 = i - t * C8;
+    const int across = BWD ? W : Wo, down = BWD ? H : Ho;
+    const int pw = t % across;
+    t /= across;
+    const int ph = t % down, b = t / down;
+    float acc[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[j] = 0.f;
+    const uint4* base = reinterpret_cast<const uint4*>(src) + (long long)b * (BWD ? Ho * Wo : H * W) * C8 + c8;
+    auto add = [&](const uint4& q, float f) {
+      const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 v = unpack2<T>(w[j]);
+        acc[2 * j] += BWD ? v.x / f : v.x;
+        acc[2 * j + 1] += BWD ? v.y / f : v.y;
+      }
+    };
+    float count = 1.f;
+    if constexpr (!BWD) {
+      const int h0 = (ph * H) / Ho, h1 = ((ph + 1) * H + Ho - 1) / Ho;
+      const int w0 = (pw * W) / Wo, w1 = ((pw + 1) * W + Wo - 1) / Wo;
+      for (int h = h0; h < h1; ++h) {
+#pragma unroll 8
+        for (int w = w0; w < w1; ++w) add(base[(long long)(h * W + w) * C8], 1.f);
+      }
+      count = (float)((h1 - h0) * (w1 - w0));
+    } else {
+      for (int oh = 0; oh < Ho; ++oh) {
+        const int h0 = (oh * H) / Ho, h1 = ((oh + 1) * H + Ho - 1) / Ho;
+        if (ph < h0 || ph >= h1) continue;
+        for (int ow = 0; ow < Wo; ++ow) {
+          const int w0 = (ow * W) / Wo, w1 = ((ow + 1) * W + Wo - 1) / Wo;
+          if (pw >= w0 && pw < w1) add(base[(long long)(oh * Wo + ow) * C8], (float)((h1 - h0) * (w1 - w0)));
+        }
       }
     }
-    uint4 out;
-    T* oe = reinterpret_cast<T*>(&out);
+    uint32_t o[4];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) oe[j] = from_f32<T>(acc[j]);
-    *reinterpret_cast<uint4*>(dx + i * 8) = out;
+    for (int j = 0; j < 4; ++j) o[j] = pack2<T>(BWD ? acc[2 * j] : acc[2 * j] / count, BWD ? acc[2 * j + 1] : acc[2 * j + 1] / count);
+    reinterpret_cast<uint4*>(dst)[i] = make_uint4(o[0], o[1], o[2], o[3]);
   }
 }
 // adaptive average pool, bins [floor(o*H/Ho), ceil((o+1)*H/Ho))
@@ -823,7 +941,7 @@ int rb_bn_fwd(int dtype, const void* x, const void* res, const void* gamma, cons
     if (vec8) {
       dim3 grid(cg / cgb, slabs);
       RB_DISPATCH_16(dtype, (bn_partial_vec8_kernel<T, false><<<grid, 256, 0, st>>>((const T*)x, nullptr, nullptr, nullptr, nullptr, scratch, M, C, rps, 0, cgb)));
-      bn_finalize_fwd_par_kernel<<<(C + 31) / 32, 256, 0, st>>>(scratch, slabs, C, M, eps, momentum, mean, rstd, running_mean, running_var);
+      bn_finalize_fwd_par_kernel<<<(C + kBnFoldCols - 1) / kBnFoldCols, 256, 0, st>>>(scratch, slabs, C, M, eps, momentum, mean, rstd, running_mean, running_var);
     } else {
       dim3 grid((C + 63) / 64, slabs);
       RB_DISPATCH_T(dtype, (bn_partial_kernel<T, false><<<grid, 64, 0, st>>>((const T*)x, nullptr, nullptr, nullptr, nullptr, scratch, M, C, rps, 0)));
@@ -855,7 +973,7 @@ int rb_bn_bwd(int dtype, const void* x, const void* dy, const void* y, const voi
     const int cgb = cg < 32 ? cg : 32;
     dim3 grid(cg / cgb, slabs);
     RB_DISPATCH_16(dtype, (bn_partial_vec8_kernel<T, true><<<grid, 256, 0, st>>>((const T*)x, (const T*)dy, (const T*)y, mean, rstd, scratch, M, C, rps, relu, cgb)));
-    RB_DISPATCH_16(dtype, (bn_finalize_bwd_par_kernel<T><<<(C + 31) / 32, 256, 0, st>>>(scratch, slabs, C, sums, (T*)dgamma, (T*)dbeta)));
+    RB_DISPATCH_16(dtype, (bn_finalize_bwd_par_kernel<T><<<(C + kBnFoldCols - 1) / kBnFoldCols, 256, 0, st>>>(scratch, slabs, C, sums, (T*)dgamma, (T*)dbeta)));
     RB_DISPATCH_16(dtype, (bn_bwd_apply_vec8_kernel<T><<<bn_grid(M * cg), 256, 0, st>>>((const T*)x, (const T*)dy, (const T*)y, (const T*)gamma, mean, rstd, sums, (T*)dx, (T*)dres, M * cg, C, M, relu, training)));
     RB_RET_LAST();
   }
@@ -871,6 +989,17 @@ int rb_maxpool_fwd(int dtype, const void* x, void* y, signed char* idx, int B, i
   cudaStream_t st = (cudaStream_t)stream;
   const long long n = (long long)B * Ho * Wo * C;
   if (n <= 0) return 0;
+  const bool vec8 = dtype != rbh::DT_F32 && C % 8 == 0 && n / 8 < (1ll << 31) && (long long)H * W * C < (1ll << 31) &&
+                    ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0 &&
+                    (reinterpret_cast<uintptr_t>(idx) & 7) == 0;
+  if (vec8) {
+#define RB_MP(KS) RB_DISPATCH_16(dtype, (maxpool_nhwc_fwd_vec8_kernel<T, KS><<<vgrid(n / 8), 256, 0, st>>>((const T*)x, (T*)y, idx, B, H, W, C / 8, K, stride, pad, Ho, Wo)))
+    if (K == 3) { RB_MP(3); }
+    else if (K == 2) { RB_MP(2); }
+    else { RB_MP(0); }
+#undef RB_MP
+    RB_RET_LAST();
+  }
   RB_DISPATCH_T(dtype, (maxpool_nhwc_fwd_kernel<T><<<vgrid(n), 256, 0, st>>>((const T*)x, (T*)y, idx, B, H, W, C, K, stride, pad, Ho, Wo)));
   RB_RET_LAST();
 }
@@ -880,14 +1009,11 @@ int rb_maxpool_bwd(int dtype, const void* dy, const signed char* idx, void* dx, 
   cudaStream_t st = (cudaStream_t)stream;
   const long long n = (long long)B * H * W * C;
   if (n <= 0) return 0;
-  const bool vec8 = dtype != rbh::DT_F32 && C % 8 == 0 &&
+  const bool vec8 = dtype != rbh::DT_F32 && C % 8 == 0 && n / 8 < (1ll << 31) &&
                     ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(dx)) & 15) == 0 &&
                     (reinterpret_cast<uintptr_t>(idx) & 7) == 0;
   if (vec8) {
-    if (dtype == rbh::DT_BF16)
-      maxpool_nhwc_bwd_vec8_kernel<__nv_bfloat16><<<vgrid(n / 8), 256, 0, st>>>((const __nv_bfloat16*)dy, idx, (__nv_bfloat16*)dx, B, H, W, C, K, stride, pad, Ho, Wo);
-    else
-      maxpool_nhwc_bwd_vec8_kernel<__half><<<vgrid(n / 8), 256, 0, st>>>((const __half*)dy, idx, (__half*)dx, B, H, W, C, K, stride, pad, Ho, Wo);
+    RB_DISPATCH_16(dtype, (maxpool_nhwc_bwd_vec8_kernel<T><<<vgrid(n / 8), 256, 0, st>>>((const T*)dy, idx, (T*)dx, B, H, W, C / 8, K, stride, pad, Ho, Wo)));
     RB_RET_LAST();
   }
   RB_DISPATCH_T(dtype, (maxpool_nhwc_bwd_kernel<T><<<vgrid(n), 256, 0, st>>>((const T*)dy, idx, (T*)dx, B, H, W, C, K, stride, pad, Ho, Wo)));
@@ -899,6 +1025,16 @@ int rb_adaptive_avgpool(int dtype, int backward, const void* src, void* dst, int
   cudaStream_t st = (cudaStream_t)stream;
   const long long n = backward ? (long long)B * H * W * C : (long long)B * Ho * Wo * C;
   if (n <= 0) return 0;
+  const bool vec8 = dtype != rbh::DT_F32 && C % 8 == 0 && n / 8 < (1ll << 31) &&
+                    ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0;
+  if (vec8) {
+    if (backward) {
+      RB_DISPATCH_16(dtype, (adaptive_avgpool_nhwc_vec8_kernel<T, true><<<vgrid(n / 8), 256, 0, st>>>((const T*)src, (T*)dst, B, H, W, C / 8, Ho, Wo)));
+    } else {
+      RB_DISPATCH_16(dtype, (adaptive_avgpool_nhwc_vec8_kernel<T, false><<<vgrid(n / 8), 256, 0, st>>>((const T*)src, (T*)dst, B, H, W, C / 8, Ho, Wo)));
+    }
+    RB_RET_LAST();
+  }
   if (backward) {
     RB_DISPATCH_T(dtype, (adaptive_avgpool_nhwc_kernel<T, true><<<vgrid(n), 256, 0, st>>>((const T*)src, (T*)dst, B, H, W, C, Ho, Wo)));
   } else {
