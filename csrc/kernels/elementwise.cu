@@ -295,7 +295,7 @@ __global__ void colsum_partial_kernel(const T* __restrict__ x, float* __restrict
   for (long long r = r0; r < r1; ++r) acc += to_f32<T>(x[r * ld + c]);
   partials[(long long)blockIdx.y * N + c] = acc;
 }
-// vector variant: each thread owns VEC consecutive columns (16-byte loads), 4 rows in flight
+// vector variant: each thread owns VEC consecutive columns (16-byte loads), 16 rows in flight
 template <typename T>
 __global__ void __launch_bounds__(128)
     colsum_partial_vec_kernel(const T* __restrict__ x, float* __restrict__ partials, long long rows,
@@ -309,12 +309,12 @@ __global__ void __launch_bounds__(128)
 #pragma unroll
   for (int j = 0; j < VEC; ++j) acc[j] = 0.f;
   long long r = r0;
-  for (; r + 4 <= r1; r += 4) {
-    uint4 v[4];
+  for (; r + 16 <= r1; r += 16) {
+    uint4 v[16];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) v[u] = *reinterpret_cast<const uint4*>(x + (r + u) * ld + c);
+    for (int u = 0; u < 16; ++u) v[u] = *reinterpret_cast<const uint4*>(x + (r + u) * ld + c);
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < 16; ++u) {
       const T* e = reinterpret_cast<const T*>(&v[u]);
 #pragma unroll
       for (int j = 0; j < VEC; ++j) acc[j] += to_f32<T>(e[j]);

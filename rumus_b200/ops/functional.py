@@ -106,10 +106,32 @@ def _wgrad(x2, dy2, mg):
     return None
 
 
+def _target(mg, like):
+    """The arena's own place for a small gradient when a kernel may write it there: the first gradient of a step, of the
+    parameter's type.  None: it goes through ``_small_grad``."""
+    if mg is None:
+        return None
+    buf, p = mg
+    if getattr(p, "grad_accumulate", False) or buf.dtype != like.dtype or buf.device != like.device or not buf.is_contiguous():
+        return None
+    return buf
+
+
+def _written(g, mg, target):
+    """What autograd gets for a gradient that a kernel wrote to ``target`` (or, without one, to ``g``)."""
+    if target is None:
+        return _small_grad(g, mg)
+    mg[1].grad_accumulate = True
+    return None
+
+
 def _bgrad(dy2, mg):
-    g = native.colsum(dy2)
+    target = _target(mg, dy2)
+    g = native.colsum(dy2, out=target)
     if mg is None:
         return g
+    if target is not None:
+        return _written(g, mg, target)
     buf, p = mg
     if getattr(p, "grad_accumulate", False):
         buf.add_(g)
@@ -328,10 +350,10 @@ class _NormFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy, dh):
         xn, gamma, stats = ctx.saved_tensors
-        dx, dg, db = native.norm_bwd(xn, dy, gamma, stats, ctx.rms, dres=dh,
-                                     want_beta=ctx.has_beta)
-        dg = _small_grad(dg, ctx.mg[0])
-        db = _small_grad(db, ctx.mg[1]) if ctx.has_beta else None
+        tg, tb = _target(ctx.mg[0], gamma), _target(ctx.mg[1], gamma)
+        dx, dg, db = native.norm_bwd(xn, dy, gamma, stats, ctx.rms, dres=dh, want_beta=ctx.has_beta, dgamma=tg, dbeta=tb)
+        dg = _written(dg, ctx.mg[0], tg)
+        db = _written(db, ctx.mg[1], tb) if ctx.has_beta else None
         return dx, dg, db, (dx if ctx.has_res else None), None, None
 
 
@@ -353,9 +375,10 @@ class _NormSkipFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy, dskip):
         x, gamma, stats = ctx.saved_tensors
-        dx, dg, db = native.norm_bwd(x, dy, gamma, stats, ctx.rms, dres=dskip, want_beta=ctx.has_beta)
-        dg = _small_grad(dg, ctx.mg[0])
-        db = _small_grad(db, ctx.mg[1]) if ctx.has_beta else None
+        tg, tb = _target(ctx.mg[0], gamma), _target(ctx.mg[1], gamma)
+        dx, dg, db = native.norm_bwd(x, dy, gamma, stats, ctx.rms, dres=dskip, want_beta=ctx.has_beta, dgamma=tg, dbeta=tb)
+        dg = _written(dg, ctx.mg[0], tg)
+        db = _written(db, ctx.mg[1], tb) if ctx.has_beta else None
         return dx, dg, db, None, None
 
 

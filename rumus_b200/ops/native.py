@@ -346,8 +346,9 @@ def norm_fwd(x, gamma, beta, eps, rms: bool, residual=None):
     return y.view(x.shape), (h.view(x.shape) if h is not None else None), stats
 
 
-def norm_bwd(xn, dy, gamma, stats, rms: bool, dres=None, want_beta=True):
-    """xn: the tensor that was normalised (x, or x+residual)."""
+def norm_bwd(xn, dy, gamma, stats, rms: bool, dres=None, want_beta=True, dgamma=None, dbeta=None):
+    """xn: the tensor that was normalised (x, or x+residual).  ``dgamma``, ``dbeta``: contiguous tensors of gamma's type to
+    write the parameters' gradients into (else new ones)."""
     L = _L()
     D = xn.shape[-1]
     x2 = xn.reshape(-1, D)
@@ -361,8 +362,12 @@ def norm_bwd(xn, dy, gamma, stats, rms: bool, dres=None, want_beta=True):
         if not dr2.is_contiguous():
             dr2 = dr2.contiguous()
     dx = torch.empty_like(x2)
-    dgamma = torch.empty_like(gamma)
-    dbeta = torch.empty_like(gamma) if (want_beta and not rms) else None
+    if dgamma is None:
+        dgamma = torch.empty_like(gamma)
+    if not want_beta or rms:
+        dbeta = None
+    elif dbeta is None:
+        dbeta = torch.empty_like(gamma)
     nparts = L.rb_norm_bwd_partials(rows)
     scratch = torch.empty((nparts, 2, D), dtype=torch.float32, device=xn.device)
     rc = L.rb_norm_bwd(dtype_code(xn.dtype), 1 if rms else 0, ptr(x2), ptr(dy2), ptr(gamma),
@@ -535,14 +540,15 @@ def rope_(x2d, tokens: int, seq_len: int, heads: int, head_dim: int, col0: int, 
     return x2d
 
 
-def colsum(x2d):
-    """Column sums of a [rows, N] matrix (bias gradient)."""
+def colsum(x2d, out=None):
+    """Column sums of a [rows, N] matrix (bias gradient); ``out``: contiguous ``[N]`` tensor of its type to write into."""
     L = _L()
     assert x2d.dim() == 2 and x2d.stride(1) == 1
     rows, N = x2d.shape
     slabs = L.rb_colsum_slabs(rows)
     scratch = torch.empty((slabs, N), dtype=torch.float32, device=x2d.device)
-    out = torch.empty(N, dtype=x2d.dtype, device=x2d.device)
+    if out is None:
+        out = torch.empty(N, dtype=x2d.dtype, device=x2d.device)
     check(L.rb_colsum(dtype_code(x2d.dtype), ptr(x2d), ptr(out), ptr(scratch), rows, N,
                       x2d.stride(0) if rows > 1 else N, stream_ptr()), "rb_colsum")
     count_launch(2)
