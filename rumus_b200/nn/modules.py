@@ -18,6 +18,7 @@ import torch
 import torch.nn as nn
 
 from ..ops import functional as F
+from ..ops.attention import f32_covered
 
 
 class Module(nn.Module):
@@ -209,6 +210,9 @@ class MultiheadAttention(Module):
         q = q.view(B, S, H, hd)
         k = k.view(B, S, Hkv, hd)
         v = v.view(B, S, Hkv, hd)
+        if mask is None and qkv.is_contiguous() and qkv.data_ptr() % 16 == 0 and f32_covered(q, k, v, self.causal):
+            o = F.flash_attention_packed(qkv, H, Hkv, self.causal)
+            return self.out_proj(o.reshape(B, S, self.d_model), residual=residual)
         if mask is not None:
             # additive-mask path of the reference API (materialised scores)
             qh = q.permute(0, 2, 1, 3).reshape(B * H, S, hd)

@@ -16,6 +16,8 @@ native.register_signature("rb_flash_attn_fwd", [I, I, P, P, P, P, P, P, P, P, I,
 native.register_signature("rb_flash_attn_bwd", [I, I, P, P, P, P, P, P, P, P, P, P, P, P, P, P, P,
                                                 I, I, I, I, I, I, F, P])
 native.register_signature("rb_fa_dq_cast", [I, P, P, P, I, I, I, P])
+native.register_signature("rb_attn_f32_fwd", [I] + [P] * 8 + [I] * 5 + [F, P])
+native.register_signature("rb_attn_f32_bwd", [I] + [P] * 16 + [I] * 5 + [F, P])
 
 
 def _strides3(t: torch.Tensor):
@@ -28,6 +30,42 @@ def _strides3(t: torch.Tensor):
 def _tma_ok(t: torch.Tensor) -> bool:
     return (t.stride(3) == 1 and t.data_ptr() % 16 == 0
             and all((t.stride(i) * t.element_size()) % 16 == 0 for i in range(3)))
+
+
+F32_MAX_ROWS = 1024
+
+
+def f32_covered(q, k, v, causal: bool) -> bool:
+    """Whether the 32-bit kernels (``csrc/kernels/attn_f32.cu``) take these heads: as many key heads as query heads, a key for
+    every row.  Sequences beyond ``F32_MAX_ROWS`` stay with the batched products."""
+    (_, Sq, H, D), (_, Sk, Hkv, _) = q.shape, k.shape
+    return (q.is_cuda and q.dtype == k.dtype == v.dtype == torch.float32 and D in (16, 32, 64, 128) and H == Hkv and 0 < Sk <= F32_MAX_ROWS
+            and 0 < Sq and (Sk >= Sq or not causal) and v.shape == k.shape)
+
+
+def attn_f32_forward(q, k, v, causal: bool, scale: float):
+    B, Sq, H, D = q.shape
+    q, k, v = (t if _tma_ok(t) else t.contiguous() for t in (q, k, v))
+    o = torch.empty((B, Sq, H, D), dtype=torch.float32, device=q.device)
+    lse = torch.empty((B, H, Sq), dtype=torch.float32, device=q.device)
+    st = [_strides3(t) for t in (q, k, v)]
+    check(native.lib().rb_attn_f32_fwd(D, ptr(q), ptr(k), ptr(v), *map(ctypes.addressof, st), ptr(o), ptr(lse), B, H, Sq, k.shape[1],
+                                       int(causal), float(scale), stream_ptr()), "rb_attn_f32_fwd")
+    count_launch()
+    return o, lse, (q, k, v)
+
+
+def attn_f32_backward(q, k, v, o, lse, dout, causal: bool, scale: float, out):
+    """``out``: dq, dk, dv of the shapes of q, k, v, rows of numbers side by side."""
+    B, Sq, H, D = q.shape
+    if not _tma_ok(dout):
+        dout = dout.contiguous()
+    dq, dk, dv = out
+    st, dst = [_strides3(t) for t in (q, k, v, dout)], [_strides3(t) for t in out]
+    check(native.lib().rb_attn_f32_bwd(D, ptr(q), ptr(k), ptr(v), ptr(o), ptr(dout), ptr(lse), *map(ctypes.addressof, st), ptr(dq), ptr(dk),
+                                       ptr(dv), *map(ctypes.addressof, dst), B, H, Sq, k.shape[1], int(causal), float(scale),
+                                       stream_ptr()), "rb_attn_f32_bwd")
+    count_launch()
 
 
 def fa_forward(q, k, v, causal: bool, scale: float, out=None):
@@ -66,7 +104,8 @@ def fa_backward(q, k, v, o, lse, dout, causal: bool, scale: float, out=None):
         dq, dk, dv = out
     assert dk.stride() == dv.stride() and dk.stride(3) == 1 and dq.stride(3) == 1
     sq_pad = (Sq + 63) // 64 * 64
-    stats = torch.zeros((2, B, H, sq_pad), dtype=torch.float32, device=q.device)  # delta | lse*log2e
+    # delta | lse * log2 e; only rows of padding have to be cleared, the kernel writes all others
+    stats = (torch.empty if sq_pad == Sq else torch.zeros)((2, B, H, sq_pad), dtype=torch.float32, device=q.device)
     qs, ks, vs, dos = _strides3(q), _strides3(k), _strides3(v), _strides3(dout)
     dkvs, dqs = _strides3(dk), _strides3(dq)
     rc = L.rb_flash_attn_bwd(native.dtype_code(q.dtype), D, ptr(q), ptr(k), ptr(v), ptr(o),
@@ -100,17 +139,42 @@ class _FlashAttnFn(torch.autograd.Function):
         return dq, dk, dv, None, None
 
 
+class _AttnF32Fn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, q, k, v, causal, scale):
+        o, lse, (qc, kc, vc) = attn_f32_forward(q, k, v, causal, scale)
+        ctx.causal, ctx.scale = causal, scale
+        ctx.save_for_backward(qc, kc, vc, o, lse)
+        return o
+
+    @staticmethod
+    def backward(ctx, dout):
+        q, k, v, o, lse = ctx.saved_tensors
+        out = [torch.empty(t.shape, dtype=t.dtype, device=t.device) for t in (q, k, v)]
+        attn_f32_backward(q, k, v, o, lse, dout, ctx.causal, ctx.scale, out)
+        return (*out, None, None)
+
+
+def attention_f32(q, k, v, causal: bool = True, scale: Optional[float] = None):
+    """32-bit attention by one kernel forward and one backward; for what ``f32_covered`` takes."""
+    return _AttnF32Fn.apply(q, k, v, causal, scale if scale is not None else 1.0 / math.sqrt(q.shape[-1]))
+
+
 class _FlashAttnPackedFn(torch.autograd.Function):
-    """Attention on the packed projection output ``qkv [B, S, (H + 2*Hkv) * 128]``: the backward
+    """Attention on the packed projection output ``qkv [B, S, (H + 2*Hkv) * hd]``: the backward
     kernels write d_q, d_k, d_v into the three slices of one d_qkv buffer (no concatenation)."""
 
     @staticmethod
-    def forward(ctx, qkv, heads, kv_heads, causal, scale):
-        B, S, _ = qkv.shape
-        hd = 128
+    def _heads(qkv, heads, kv_heads):
+        B, S, n = qkv.shape
+        hd = n // (heads + 2 * kv_heads)
         q, k, v = qkv.split([heads * hd, kv_heads * hd, kv_heads * hd], dim=-1)
-        q, k, v = q.view(B, S, heads, hd), k.view(B, S, kv_heads, hd), v.view(B, S, kv_heads, hd)
-        o, lse, _ = fa_forward(q, k, v, causal, scale)
+        return q.view(B, S, heads, hd), k.view(B, S, kv_heads, hd), v.view(B, S, kv_heads, hd)
+
+    @staticmethod
+    def forward(ctx, qkv, heads, kv_heads, causal, scale):
+        q, k, v = _FlashAttnPackedFn._heads(qkv, heads, kv_heads)
+        o, lse, _ = (attn_f32_forward if qkv.dtype == torch.float32 else fa_forward)(q, k, v, causal, scale)
         ctx.causal, ctx.scale, ctx.heads, ctx.kv_heads = causal, scale, heads, kv_heads
         ctx.save_for_backward(qkv, o, lse)
         return o
@@ -118,23 +182,19 @@ class _FlashAttnPackedFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dout):
         qkv, o, lse = ctx.saved_tensors
-        B, S, _ = qkv.shape
-        H, Hkv, hd = ctx.heads, ctx.kv_heads, 128
-        sizes = [H * hd, Hkv * hd, Hkv * hd]
-        q, k, v = qkv.split(sizes, dim=-1)
-        q, k, v = q.view(B, S, H, hd), k.view(B, S, Hkv, hd), v.view(B, S, Hkv, hd)
         dqkv = torch.empty_like(qkv)
-        dq, dk, dv = dqkv.split(sizes, dim=-1)
-        out = (dq.view(B, S, H, hd), dk.view(B, S, Hkv, hd), dv.view(B, S, Hkv, hd))
-        fa_backward(q, k, v, o, lse, dout, ctx.causal, ctx.scale, out=out)
+        q, k, v = _FlashAttnPackedFn._heads(qkv, ctx.heads, ctx.kv_heads)
+        out = _FlashAttnPackedFn._heads(dqkv, ctx.heads, ctx.kv_heads)
+        (attn_f32_backward if qkv.dtype == torch.float32 else fa_backward)(q, k, v, o, lse, dout, ctx.causal, ctx.scale, out=out)
         return dqkv, None, None, None, None
 
 
 def flash_attention_packed(qkv, heads: int, kv_heads: int, causal: bool = True,
                            scale: Optional[float] = None):
-    """``qkv`` is the fused projection output, head_dim 128, CUDA, 16-bit, 16-byte aligned rows."""
+    """``qkv`` is the fused projection output on a GPU, 16-byte aligned rows: 16-bit with head_dim 128, or 32-bit with heads that
+    ``f32_covered`` takes."""
     if scale is None:
-        scale = 1.0 / math.sqrt(128)
+        scale = 1.0 / math.sqrt(qkv.shape[-1] // (heads + 2 * kv_heads))
     return _FlashAttnPackedFn.apply(qkv, heads, kv_heads, causal, scale)
 
 

@@ -671,6 +671,9 @@ def flash_attention(q, k, v, causal: bool = True, scale: Optional[float] = None)
         from .attention import flash_attention_cuda
         return flash_attention_cuda(q, k, v, causal, scale)
     if _is_native(q):
+        from .attention import attention_f32, f32_covered
+        if f32_covered(q, k, v, causal):
+            return attention_f32(q, k, v, causal, scale)
         return _sdpa_composed(q, k, v, causal, scale)
     return sdpa_reference(q, k, v, causal, scale)
 
