@@ -680,9 +680,10 @@ int launch_norm_fwd(const void* x, const void* res, const void* gamma, const voi
   norm_fwd_kernel<T, RMS, IT><<<(unsigned)blocks, kNormWarps * 32, 0, st>>>(                       \
       (const T*)x, (const T*)res, (const T*)gamma, (const T*)beta, (T*)y, (T*)h_out, stats, rows, \
       D, eps)
-  // rows of more than four vectors a lane: a CTA per row, as many threads as vectors up to 256
+  // RMS norms of more than four vectors a lane: a CTA per row, as many threads as vectors up to 256.  (Layer norms are met in
+  // training, where there are rows enough for a warp each; another order of their sums would move a step's gradients by rounding.)
   const int vecs = D / VEC;
-  if (vec && iters > 4 && vecs <= 4 * 256 && rows < (1ll << 31)) {
+  if (RMS && vec && iters > 4 && vecs <= 4 * 256 && rows < (1ll << 31)) {
     const int per = (vecs + 255) / 256;
     const int threads = ((vecs + per - 1) / per + 31) / 32 * 32;
 #define RB_NORM_WIDE(V)                                                                           \
