@@ -366,32 +366,31 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// Sums the slab partials of 8 channels (one 32-byte sector) with 32 slab slices per CTA, eight slabs of a slice in flight: what
-// counts is the chain of waits, not the bytes (up to 2048 slabs; with eight slices of 32 channels and one slab in flight 13 us).
-constexpr int kBnFoldCols = 8, kBnFoldSlices = 32;
+// Sums the slab partials of 8 channels (one 32-byte sector) with 8 slab slices per CTA, 32 slabs of a slice in flight: what counts is
+// the chain of waits, not the bytes (up to 2048 slabs; with 32 channels a CTA and one slab at a time 13 us).  The additions of
+// a slice go in the order of its slabs.
+constexpr int kBnFoldCols = 8, kBnFoldThreads = 64;
 __device__ __forceinline__ void bn_fold_partials(const float* __restrict__ partials, int slabs, int C, int c, int slice, int cx,
                                                  float& s, float& q) {
-  __shared__ float ss[kBnFoldSlices][kBnFoldCols + 1], sq[kBnFoldSlices][kBnFoldCols + 1];
+  constexpr int AHEAD = 32;
+  __shared__ float ss[8][kBnFoldCols + 1], sq[8][kBnFoldCols + 1];
   s = 0.f;
   q = 0.f;
   if (c < C) {
-    int i = slice;
-    for (; i + 7 * kBnFoldSlices < slabs; i += 8 * kBnFoldSlices) {
-      float a[8], b[8];
+    for (int i = slice; i < slabs; i += 8 * AHEAD) {
+      float a[AHEAD], b[AHEAD];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        a[u] = partials[((long long)(i + u * kBnFoldSlices) * 2) * C + c];
-        b[u] = partials[((long long)(i + u * kBnFoldSlices) * 2 + 1) * C + c];
+      for (int u = 0; u < AHEAD; ++u) {
+        const bool in = i + 8 * u < slabs;
+        const float* at = partials + ((long long)(i + 8 * u) * 2) * C + c;
+        a[u] = in ? at[0] : 0.f;
+        b[u] = in ? at[C] : 0.f;
       }
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
+      for (int u = 0; u < AHEAD; ++u) {
         s += a[u];
         q += b[u];
       }
-    }
-    for (; i < slabs; i += kBnFoldSlices) {
-      s += partials[((long long)i * 2) * C + c];
-      q += partials[((long long)i * 2 + 1) * C + c];
     }
   }
   ss[slice][cx] = s;
@@ -399,14 +398,14 @@ __device__ __forceinline__ void bn_fold_partials(const float* __restrict__ parti
   __syncthreads();
   if (slice == 0) {
 #pragma unroll
-    for (int k = 1; k < kBnFoldSlices; ++k) {
+    for (int k = 1; k < 8; ++k) {
       s += ss[k][cx];
       q += sq[k][cx];
     }
   }
 }
 
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kBnFoldThreads)
     bn_finalize_fwd_par_kernel(const float* __restrict__ partials, int slabs, int C, long long M,
                                float eps, float momentum, float* __restrict__ mean,
                                float* __restrict__ rstd, float* __restrict__ running_mean,
@@ -427,7 +426,7 @@ __global__ void __launch_bounds__(256)
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kBnFoldThreads)
     bn_finalize_bwd_par_kernel(const float* __restrict__ partials, int slabs, int C,
                                float* __restrict__ sums, T* __restrict__ dgamma,
                                T* __restrict__ dbeta) {
@@ -941,7 +940,7 @@ int rb_bn_fwd(int dtype, const void* x, const void* res, const void* gamma, cons
     if (vec8) {
       dim3 grid(cg / cgb, slabs);
       RB_DISPATCH_16(dtype, (bn_partial_vec8_kernel<T, false><<<grid, 256, 0, st>>>((const T*)x, nullptr, nullptr, nullptr, nullptr, scratch, M, C, rps, 0, cgb)));
-      bn_finalize_fwd_par_kernel<<<(C + kBnFoldCols - 1) / kBnFoldCols, 256, 0, st>>>(scratch, slabs, C, M, eps, momentum, mean, rstd, running_mean, running_var);
+      bn_finalize_fwd_par_kernel<<<(C + kBnFoldCols - 1) / kBnFoldCols, kBnFoldThreads, 0, st>>>(scratch, slabs, C, M, eps, momentum, mean, rstd, running_mean, running_var);
     } else {
       dim3 grid((C + 63) / 64, slabs);
       RB_DISPATCH_T(dtype, (bn_partial_kernel<T, false><<<grid, 64, 0, st>>>((const T*)x, nullptr, nullptr, nullptr, nullptr, scratch, M, C, rps, 0)));
@@ -973,7 +972,7 @@ int rb_bn_bwd(int dtype, const void* x, const void* dy, const void* y, const voi
     const int cgb = cg < 32 ? cg : 32;
     dim3 grid(cg / cgb, slabs);
     RB_DISPATCH_16(dtype, (bn_partial_vec8_kernel<T, true><<<grid, 256, 0, st>>>((const T*)x, (const T*)dy, (const T*)y, mean, rstd, scratch, M, C, rps, relu, cgb)));
-    RB_DISPATCH_16(dtype, (bn_finalize_bwd_par_kernel<T><<<(C + kBnFoldCols - 1) / kBnFoldCols, 256, 0, st>>>(scratch, slabs, C, sums, (T*)dgamma, (T*)dbeta)));
+    RB_DISPATCH_16(dtype, (bn_finalize_bwd_par_kernel<T><<<(C + kBnFoldCols - 1) / kBnFoldCols, kBnFoldThreads, 0, st>>>(scratch, slabs, C, sums, (T*)dgamma, (T*)dbeta)));
     RB_DISPATCH_16(dtype, (bn_bwd_apply_vec8_kernel<T><<<bn_grid(M * cg), 256, 0, st>>>((const T*)x, (const T*)dy, (const T*)y, (const T*)gamma, mean, rstd, sums, (T*)dx, (T*)dres, M * cg, C, M, relu, training)));
     RB_RET_LAST();
   }
