@@ -60,7 +60,8 @@ __global__ void __launch_bounds__(256)
       v = apply_act(v, p.act);
       if (p.aux_in)
         v *= apply_dact(to_f32<OT>(reinterpret_cast<const OT*>(p.aux_in)[m * p.ldaux_in + n]), p.dact);
-      if (p.residual) v += to_f32<OT>(reinterpret_cast<const OT*>(p.residual)[m * p.ldr + n]);
+      if (p.residual)
+        v = (p.round_first ? to_f32<OT>(from_f32<OT>(v)) : v) + to_f32<OT>(reinterpret_cast<const OT*>(p.residual)[m * p.ldr + n]);
       out[m * p.ldc + n] = from_f32<OT>(v);
     }
   }
@@ -105,7 +106,7 @@ int rb_gemm(int dtype, int a_mn, int b_mn, const void* A, long long lda, const v
   GemmParams& p = a.p;
   p.M = M; p.N = N; p.K = K; p.out = out; p.bias = bias; p.residual = residual;
   p.aux_out = aux_out; p.aux_in = aux_in; p.ldc = ldc; p.ldr = ldr; p.ldaux_out = ldaux_out;
-  p.ldaux_in = ldaux_in; p.act = act; p.dact = dact; p.out_f32 = out_f32; p.alpha = alpha;
+  p.ldaux_in = ldaux_in; p.act = act & 0xff; p.round_first = act & ACT_ROUND_FIRST; p.dact = dact; p.out_f32 = out_f32; p.alpha = alpha;
   p.status = rbh::device_status_word();
   p.group_m = 8;
   p.split_k = 1;

@@ -127,7 +127,7 @@ int rb_gemm_2cta(int dtype, int a_mn, int b_mn, const void* A, long long lda, co
   GemmParams& p = a.p;
   p.M = M; p.N = N; p.K = K; p.out = out; p.bias = bias; p.residual = residual;
   p.aux_out = aux_out; p.aux_in = aux_in; p.ldc = ldc; p.ldr = ldr; p.ldaux_out = ldaux_out;
-  p.ldaux_in = ldaux_in; p.act = act; p.dact = dact; p.out_f32 = out_f32; p.alpha = alpha;
+  p.ldaux_in = ldaux_in; p.act = act & 0xff; p.round_first = act & ACT_ROUND_FIRST; p.dact = dact; p.out_f32 = out_f32; p.alpha = alpha;
   p.status = rbh::device_status_word();
   p.split_k = 1;
   p.sched = rbh::dynamic_tiles() ? rbh::next_sched_slot() : nullptr;

@@ -171,7 +171,7 @@ __device__ __forceinline__ void epilogue_math32(const GemmParams& p, const uint3
     float r[32];
     load_row32<OT>(reinterpret_cast<const OT*>(p.residual), p.ldr, row, col, ncols_valid, vec, r);
 #pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] += r[i];
+    for (int i = 0; i < 32; ++i) v[i] = (p.round_first ? to_f32<OT>(from_f32<OT>(v[i])) : v[i]) + r[i];
   }
 }
 
@@ -220,7 +220,7 @@ __device__ __forceinline__ void lean_pack32(const GemmParams& p, const uint32_t*
         const uint4 q = *(reinterpret_cast<const uint4*>(rs) + g);
         const T* e = reinterpret_cast<const T*>(&q);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) f[i] += to_f32<T>(e[i]);
+        for (int i = 0; i < 8; ++i) f[i] = (p.round_first ? to_f32<T>(from_f32<T>(f[i])) : f[i]) + to_f32<T>(e[i]);
       }
 #pragma unroll
       for (int i = 0; i < 4; ++i) pk[g * 4 + i] = pack2<T>(f[2 * i], f[2 * i + 1]);
@@ -232,11 +232,11 @@ __device__ __forceinline__ void lean_pack32(const GemmParams& p, const uint32_t*
       float f0 = __uint_as_float(acc_bits[2 * i]) * p.alpha, f1 = __uint_as_float(acc_bits[2 * i + 1]) * p.alpha;
       if (2 * i < ncols_valid) {
         if (b) f0 += to_f32<T>(b[2 * i]);
-        if (rs) f0 += to_f32<T>(rs[2 * i]);
+        if (rs) f0 = (p.round_first ? to_f32<T>(from_f32<T>(f0)) : f0) + to_f32<T>(rs[2 * i]);
       }
       if (2 * i + 1 < ncols_valid) {
         if (b) f1 += to_f32<T>(b[2 * i + 1]);
-        if (rs) f1 += to_f32<T>(rs[2 * i + 1]);
+        if (rs) f1 = (p.round_first ? to_f32<T>(from_f32<T>(f1)) : f1) + to_f32<T>(rs[2 * i + 1]);
       }
       pk[i] = pack2<T>(f0, f1);
     }

@@ -10,6 +10,17 @@ import torch
 import torch.nn as nn
 
 from ..nn import AdaptiveAvgPool2d, BatchNorm2d, Conv2d, Flatten, Linear, MaxPool2d, Module
+from ..ops.vision import conv2d_skip
+
+
+def conv_and_skip(conv, x):
+    """``(conv(x), x)`` with the gradients of both uses of ``x`` added in the convolution's own product; a module that is not
+    a plain ``Conv2d``, or that somebody listens to, is called as usual."""
+    hooked = (conv._forward_hooks or conv._forward_pre_hooks or conv._backward_hooks or conv._backward_pre_hooks
+              or "forward" in conv.__dict__ or torch.nn.modules.module._has_any_global_hook())
+    if type(conv) is not Conv2d or hooked:
+        return conv(x), x
+    return conv2d_skip(x, conv.weight4d(), conv.bias, conv.stride, conv.padding, conv.dilation)
 
 
 class Bottleneck(Module):
@@ -31,10 +42,10 @@ class Bottleneck(Module):
                 "bn": BatchNorm2d(out_ch, device=device, dtype=dtype)})
 
     def forward(self, x):
-        idt = x
+        y, idt = conv_and_skip(self.conv1, x)
+        y = self.bn1(y, relu=True)
         if self.downsample is not None:
-            idt = self.downsample["bn"](self.downsample["conv"](x))
-        y = self.bn1(self.conv1(x), relu=True)
+            idt = self.downsample["bn"](self.downsample["conv"](idt))
         y = self.bn2(self.conv2(y), relu=True)
         return self.bn3(self.conv3(y), relu=True, residual=idt)
 

@@ -177,7 +177,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, bias: Optional[torch.Tensor] = Non
          aux_out: bool = False, aux_in: Optional[torch.Tensor] = None, dact: Optional[str] = None,
          out_dtype: Optional[torch.dtype] = None, alpha: float = 1.0,
          out: Optional[torch.Tensor] = None, path: int = 0, bn: int = 0, max_ctas: int = 0,
-         split_k: int = 0, mt: int = 0):
+         split_k: int = 0, mt: int = 0, round_first: bool = False):
     """``out = dact'(aux_in) * act(alpha * a @ b + bias) + residual``.
 
     ``a`` is logical [M,K], ``b`` logical [K,N]; either may be a transposed view
@@ -233,7 +233,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, bias: Optional[torch.Tensor] = Non
         assert residual.dtype == odt and residual.shape == (M, N) and residual.stride(1) == 1
     if aux_in is not None:
         assert aux_in.dtype == odt and aux_in.shape == (M, N) and aux_in.stride(1) == 1
-    few = M <= 128 and not at and bt and a.dtype == torch.bfloat16 and not aux_out and aux_in is None and dact is None
+    act_code = ACT_CODES[act] | (0x100 if round_first else 0)
+    few = M <= 128 and not round_first and not at and bt and a.dtype == torch.bfloat16 and not aux_out and aux_in is None and dact is None
     # more than 32 rows: only where 128-row tiles of the weight leave most SMs idle
     if path == 4 or (path == 0 and few and (M <= 32 or (M <= 64 and N < 8192)) and N * K >= 1 << 16 and split_k == 0 and bn == 0
                      and max_ctas == 0):
@@ -248,7 +249,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, bias: Optional[torch.Tensor] = Non
         if path == 4:
             raise ValueError("operands are outside what the few-rows GEMM covers")
     plain = bias is None and act is None and not aux_out and aux_in is None and dact is None
-    if split_k == 0 and plain and path != 2 and K >= 4096:
+    if split_k == 0 and plain and not round_first and path != 2 and K >= 4096:
         tiles = ((M + 127) // 128) * ((N + 127) // 128)
         sms = sm_count()
         if tiles * 2 <= sms:
@@ -271,7 +272,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, bias: Optional[torch.Tensor] = Non
         rc = L.rb_gemm_2cta(dt, a_mn, b_mn, ptr(a), lda, ptr(b), ldb, M, N, K, ptr(out), out.stride(0),
                             out_f32, ptr(bias), ptr(residual),
                             residual.stride(0) if residual is not None else 0, ptr(pre), N, ptr(aux_in),
-                            aux_in.stride(0) if aux_in is not None else 0, ACT_CODES[act], ACT_CODES[dact],
+                            aux_in.stride(0) if aux_in is not None else 0, act_code, ACT_CODES[dact],
                             float(alpha), max_ctas, mt, stream_ptr())
         if rc != 13:
             check(rc, "rb_gemm_2cta")
@@ -286,7 +287,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, bias: Optional[torch.Tensor] = Non
                    (residual.stride(0) if M > 1 else N) if residual is not None else 0,
                    ptr(pre), N, ptr(aux_in),
                    (aux_in.stride(0) if M > 1 else N) if aux_in is not None else 0,
-                   ACT_CODES[act], ACT_CODES[dact], float(alpha), path, bn, max_ctas, 1,
+                   act_code, ACT_CODES[dact], float(alpha), path, bn, max_ctas, 1,
                    ctypes.addressof(used), stream_ptr())
     check(rc, "rb_gemm")
     count_launch()

@@ -28,6 +28,16 @@ def conv2d(x, weight, bias=None, stride: int = 1, padding: int = 0, dilation: in
     return Conv2dFn.apply(x, weight, bias, stride, padding, dilation)
 
 
+def conv2d_skip(x, weight, bias=None, stride: int = 1, padding: int = 0, dilation: int = 1):
+    """``(conv2d(x, ...), skip)``: use ``skip`` (same values as ``x``) where a block's skip connection reads its input."""
+    pointwise = weight.shape[2:] == (1, 1) and stride == 1 and padding == 0 and weight.shape[1] % (16 // x.element_size()) == 0
+    # (K below 4096: longer sums may be split, and their parts added in another precision)
+    if not x.is_cuda or not pointwise or bias is not None or weight.shape[0] >= 4096 or not (x.requires_grad and torch.is_grad_enabled()):
+        return conv2d(x, weight, bias, stride, padding, dilation), x
+    from .vision_cuda import Conv2dSkipFn
+    return Conv2dSkipFn.apply(x, weight)
+
+
 def conv_transpose2d(x, weight, bias=None, stride: int = 1, padding: int = 0):
     """x [B,Cin,H,W], weight [Cin,Cout,Kh,Kw]."""
     if not x.is_cuda:

@@ -276,6 +276,34 @@ class Conv2dFn(torch.autograd.Function):
         return dx, dw, db, None, None, None
 
 
+class Conv2dSkipFn(torch.autograd.Function):
+    """``(conv(x), x)`` for a 1x1 convolution without padding and stride: the second output is ``x`` itself, handed on as the skip connection.
+    Taking it from here means that ``x`` has one consumer in the graph, and the gradients that meet at a block's input are added
+    inside the data gradient's product (rounded before, as by an addition of its own) instead of by a pass over three tensors."""
+
+    @staticmethod
+    def forward(ctx, x, weight):
+        B, Cin, H, W = x.shape
+        xh = _nhwc(x)
+        wm = _weight_matrix(weight, Cin)
+        y = native.gemm(xh.view(B * H * W, Cin), wm.t())
+        ctx.save_for_backward(xh, wm)
+        return _as_nchw(y.view(B, H, W, weight.shape[0])), x.view_as(x)
+
+    @staticmethod
+    def backward(ctx, dy, dskip):
+        xh, wm = ctx.saved_tensors
+        B, H, W, Cin = xh.shape
+        dyh = _nhwc(dy).view(B * H * W, wm.shape[0])
+        dx = dw = None
+        if ctx.needs_input_grad[1]:
+            dw = native.gemm(dyh.t(), xh.view(B * H * W, Cin)).view(wm.shape[0], Cin, 1, 1)
+        if ctx.needs_input_grad[0]:
+            skip = _nhwc(dskip).view(B * H * W, Cin)
+            dx = _as_nchw(native.gemm(dyh, wm, residual=skip, round_first=True).view(B, H, W, Cin))
+        return dx, dw
+
+
 class _ConvTranspose2dFn(torch.autograd.Function):
     """y = col2im(x[M, Cin] @ W[Cin, Cout*K*K]) — the data-gradient path of a convolution."""
 
