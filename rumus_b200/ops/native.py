@@ -235,8 +235,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, bias: Optional[torch.Tensor] = Non
         assert aux_in.dtype == odt and aux_in.shape == (M, N) and aux_in.stride(1) == 1
     act_code = ACT_CODES[act] | (0x100 if round_first else 0)
     few = M <= 128 and not round_first and not at and bt and a.dtype == torch.bfloat16 and not aux_out and aux_in is None and dact is None
-    # more than 32 rows: only where 128-row tiles of the weight leave most SMs idle
-    if path == 4 or (path == 0 and few and (M <= 32 or (M <= 64 and N < 8192)) and N * K >= 1 << 16 and split_k == 0 and bn == 0
+    # more than 32 rows: only where 128-row tiles of the weight leave half of the SMs idle, so that four CTAs or more share K
+    # (64 rows, K 2048: N 8192 12.8 us, 13.9 on the other kernel; N 11264, two CTAs, 18.2 and 15.1)
+    if path == 4 or (path == 0 and few and (M <= 32 or (M <= 64 and 2 * ((N + 127) // 128) <= sm_count())) and N * K >= 1 << 16 and split_k == 0 and bn == 0
                      and max_ctas == 0):
         rc = 13 if not few else L.rb_gemm_rows(
             dt, ptr(a), lda, ptr(b), ldb, M, N, K, ptr(out), out.stride(0) if M > 1 else N, out_f32, ptr(bias), ptr(residual),
