@@ -87,16 +87,16 @@ def have_cuda_lib() -> bool:
     return os.path.exists(_CUDA_SO)
 
 
-def stream_ptr(device=None) -> ctypes.c_void_p:
+# Addresses go to the launchers as plain numbers (every launcher's argument types are declared, so ctypes makes pointers of them): this runs
+# ten times per launch.
+def stream_ptr(device=None) -> int:
     if device is None:       # the short way: this runs once per launch
-        return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    return torch.cuda.current_stream(device).cuda_stream
 
 
-def ptr(t) -> ctypes.c_void_p:
-    if t is None:
-        return ctypes.c_void_p(0)
-    return ctypes.c_void_p(t.data_ptr())
+def ptr(t):
+    return None if t is None else t.data_ptr()
 
 
 def count_launch(n: int = 1) -> None:
