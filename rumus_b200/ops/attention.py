@@ -35,12 +35,20 @@ def _tma_ok(t: torch.Tensor) -> bool:
 F32_MAX_ROWS = 1024
 
 
+def f32_covers(q, k, v, causal: bool) -> bool:
+    """Whether heads of these shapes are what the 32-bit kernels (``csrc/kernels/attn_f32.cu``) read and write: the batch, the
+    heads and their size of k and v are q's (the kernels step through all three by q's sizes), a key for every row."""
+    if len(q) != 4 or len(k) != 4 or k != v:
+        return False
+    (B, Sq, H, D), Sk = q, k[1]
+    return k == (B, Sk, H, D) and D in (16, 32, 64, 128) and 0 < Sk <= F32_MAX_ROWS and 0 < Sq and (Sk >= Sq or not causal)
+
+
 def f32_covered(q, k, v, causal: bool) -> bool:
-    """Whether the 32-bit kernels (``csrc/kernels/attn_f32.cu``) take these heads: as many key heads as query heads, a key for
-    every row.  Sequences beyond ``F32_MAX_ROWS`` stay with the batched products."""
-    (_, Sq, H, D), (_, Sk, Hkv, _) = q.shape, k.shape
-    return (q.is_cuda and q.dtype == k.dtype == v.dtype == torch.float32 and D in (16, 32, 64, 128) and H == Hkv and 0 < Sk <= F32_MAX_ROWS
-            and 0 < Sq and (Sk >= Sq or not causal) and v.shape == k.shape)
+    """Whether the 32-bit kernels take these tensors.  All others, sequences beyond ``F32_MAX_ROWS`` among them, stay with the batched
+    products."""
+    return (q.is_cuda and q.dtype == k.dtype == v.dtype == torch.float32 and q.device == k.device == v.device
+            and f32_covers(tuple(q.shape), tuple(k.shape), tuple(v.shape), causal))
 
 
 def attn_f32_forward(q, k, v, causal: bool, scale: float):
