@@ -52,6 +52,8 @@ def f32_covered(q, k, v, causal: bool) -> bool:
 
 
 def attn_f32_forward(q, k, v, causal: bool, scale: float):
+    if not f32_covers(tuple(q.shape), tuple(k.shape), tuple(v.shape), causal):
+        raise ValueError(f"32-bit attention kernels do not take heads {tuple(q.shape)}, {tuple(k.shape)}, {tuple(v.shape)}")
     B, Sq, H, D = q.shape
     q, k, v = (t if _tma_ok(t) else t.contiguous() for t in (q, k, v))
     o = torch.empty((B, Sq, H, D), dtype=torch.float32, device=q.device)
@@ -201,8 +203,13 @@ def flash_attention_packed(qkv, heads: int, kv_heads: int, causal: bool = True,
                            scale: Optional[float] = None):
     """``qkv`` is the fused projection output on a GPU, 16-byte aligned rows: 16-bit with head_dim 128, or 32-bit with heads that
     ``f32_covered`` takes."""
+    hd = qkv.shape[-1] // (heads + 2 * kv_heads)
+    if qkv.dtype != torch.float32 and hd != 128:      # the backward kernel's only head size
+        raise ValueError(f"packed 16-bit attention has heads of 128, not {hd}")
+    if qkv.dtype == torch.float32 and (qkv.data_ptr() % 16 or not qkv.is_contiguous()):
+        qkv = qkv.clone(memory_format=torch.contiguous_format)      # the kernels move 16 bytes at a time, the gradient's rows too
     if scale is None:
-        scale = 1.0 / math.sqrt(qkv.shape[-1] // (heads + 2 * kv_heads))
+        scale = 1.0 / math.sqrt(hd)
     return _FlashAttnPackedFn.apply(qkv, heads, kv_heads, causal, scale)
 
 

@@ -1,6 +1,7 @@
 """Which shapes the attention kernels are given: their index arithmetic takes k's and v's sizes from q, so any other shape has to be
 turned away before the launch."""
 import pytest
+import torch
 
 
 @pytest.mark.parametrize("q,k,v,causal,covered", [
@@ -20,3 +21,21 @@ import pytest
 def test_32_bit_heads(q, k, v, causal, covered):
     from rumus_b200.ops.attention import f32_covers
     assert f32_covers(q, k, v, causal) is covered
+
+
+@pytest.mark.parametrize("heads,kv_heads,hd,dtype", [
+    (4, 2, 32, torch.float32),          # key heads h >= kv_heads lie beyond the rows
+    (4, 4, 24, torch.float32),
+    (2, 2, 64, torch.bfloat16),         # forward only
+])
+def test_packed_heads_that_no_kernel_takes(heads, kv_heads, hd, dtype):
+    from rumus_b200.ops import functional as F
+    with pytest.raises(ValueError):
+        F.flash_attention_packed(torch.zeros(2, 8, (heads + 2 * kv_heads) * hd, dtype=dtype), heads, kv_heads, True)
+
+
+def test_32_bit_forward_turns_other_shapes_away():
+    from rumus_b200.ops.attention import attention_f32
+    q, k = torch.zeros(4, 8, 2, 32), torch.zeros(1, 8, 2, 32)
+    with pytest.raises(ValueError):
+        attention_f32(q, k, k, True)

@@ -50,3 +50,23 @@ def test_attention_f32_packed_is_the_same_and_the_rest_is_composed():
     assert not f32_covered(q, k, v, True)
     ref = _ref(q.double(), k.double(), v.double(), True, 24 ** -0.5)
     assert ((F.flash_attention(q, k, v, True).double() - ref).norm() / ref.norm()).item() < 1e-5
+
+
+@pytest.mark.parametrize("layout", ["four bytes on", "batch second"])
+def test_packed_rows_of_other_layouts(layout):
+    from rumus_b200.ops import functional as F
+    torch.manual_seed(1)
+    B, S, H, D = 2, 33, 2, 32
+    rows = torch.randn(B, S, 3 * H * D, device="cuda")
+    if layout == "batch second":
+        qkv = rows.transpose(0, 1).contiguous().transpose(0, 1)
+    else:
+        qkv = torch.empty(rows.numel() + 1, device="cuda")[1:].view_as(rows).copy_(rows)
+    g = torch.randn(B, S, H, D, device="cuda")
+    got, want = [], []
+    for t, out in ((qkv, got), (rows, want)):
+        t.requires_grad_()
+        o = F.flash_attention_packed(t, H, H, True)
+        out += [o, torch.autograd.grad(o, t, g)[0]]
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
