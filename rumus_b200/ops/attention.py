@@ -80,9 +80,14 @@ def attn_f32_backward(q, k, v, o, lse, dout, causal: bool, scale: float, out):
 
 def fa_forward(q, k, v, causal: bool, scale: float, out=None):
     """``out``: contiguous ``[B, Sq, H, D]`` tensor to write the heads into."""
-    L = native.lib()
     B, Sq, H, D = q.shape
-    _, Sk, Hkv, _ = k.shape
+    Bk, Sk, Hkv, Dk = k.shape
+    # the kernels describe k and v by q's batch, head size and type
+    if (Bk != B or Dk != D or v.shape != k.shape or Hkv == 0 or H % Hkv or not q.dtype == k.dtype == v.dtype
+            or not q.device == k.device == v.device):
+        raise ValueError(f"attention of heads {tuple(q.shape)}, {tuple(k.shape)}, {tuple(v.shape)} ({q.dtype}, {k.dtype}, {v.dtype}; "
+                         f"{q.device}, {k.device}, {v.device})")
+    L = native.lib()
     q, k, v = (t if _tma_ok(t) else t.contiguous() for t in (q, k, v))
     o = out if out is not None else torch.empty((B, Sq, H, D), dtype=q.dtype, device=q.device)
     assert o.is_contiguous() and o.shape == q.shape and o.dtype == q.dtype

@@ -39,3 +39,18 @@ def test_32_bit_forward_turns_other_shapes_away():
     q, k = torch.zeros(4, 8, 2, 32), torch.zeros(1, 8, 2, 32)
     with pytest.raises(ValueError):
         attention_f32(q, k, k, True)
+
+
+@pytest.mark.parametrize("q,k,v,types", [
+    ((2, 8, 4, 64), (1, 8, 4, 64), (1, 8, 4, 64), "bbb"),              # k's batch
+    ((2, 8, 4, 64), (2, 8, 4, 128), (2, 8, 4, 128), "bbb"),            # its head size
+    ((2, 8, 4, 64), (2, 9, 4, 64), (2, 8, 4, 64), "bbb"),
+    ((2, 8, 4, 64), (2, 8, 3, 64), (2, 8, 3, 64), "bbb"),              # heads that cannot be shared evenly
+    ((2, 8, 4, 64), (2, 8, 0, 64), (2, 8, 0, 64), "bbb"),
+    ((2, 8, 4, 64), (2, 8, 4, 64), (2, 8, 4, 64), "bhb"),
+])
+def test_16_bit_forward_turns_other_shapes_away(q, k, v, types):
+    from rumus_b200.ops.attention import fa_forward
+    dt = {"b": torch.bfloat16, "h": torch.float16}
+    with pytest.raises(ValueError):
+        fa_forward(*(torch.zeros(s, dtype=dt[t]) for s, t in zip((q, k, v), types)), True, 0.1)
