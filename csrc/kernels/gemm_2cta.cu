@@ -75,6 +75,7 @@ int launch_gemm_2cta_flavour(GemmArgs& a, int mt) {
   const GemmParams& p = a.p;
   const bool staged16 = p.tma_store && !p.out_f32;
   const bool lean = staged16 && !p.aux_out && !p.aux_in && p.act == ACT_NONE;
+  if (p.round_first) return lean && !a.a_mn ? launch_gemm_2cta_major<T, 1, EPI_ROUND>(a) : 13;      // 13: the one-CTA kernel
   if (lean) return mt == 2 ? launch_gemm_2cta_major<T, 2, EPI_LEAN>(a) : launch_gemm_2cta_major<T, 1, EPI_LEAN>(a);
   const char* sp = getenv("RB_G2_SPECIAL");        // "0": always take the full flavour for activation epilogues
   if (staged16 && !a.a_mn && !(sp && sp[0] == '0')) {

@@ -94,9 +94,12 @@ __device__ __forceinline__ bool bar_vote_and(int id, int threads, bool pred) {
 // forward), EPI_DGELU = multiply by the tanh-GELU derivative of a stored pre-activation (the data
 // gradient of its second layer).  The specialised bodies are a few hundred instructions; the full one is
 // large enough for its instruction fetch to show in the tile time.
+// EPI_ROUND: EPI_LEAN with the product rounded to the output's type before the residual is added (ACT_ROUND_FIRST).  A flavour of its
+// own: decided at run time it made the lean epilogue larger, and 512-row tiles, whose drain nothing hides, 8 % slower for
+// everybody (2048 x 12288, K 1024: 61.4 us against 55.7; K 4096: 7 %).
 // EPI_GLU (grouped hooks): B's rows come in blocks of 32 gates, 32 ups, ...; the output has half as many columns,
 // clamped_unit(gate, up) * row_scale.
-enum { EPI_FULL = 0, EPI_LEAN = 1, EPI_GELU_AUX = 2, EPI_DGELU = 3, EPI_GLU = 4 };
+enum { EPI_FULL = 0, EPI_LEAN = 1, EPI_GELU_AUX = 2, EPI_DGELU = 3, EPI_GLU = 4, EPI_ROUND = 5 };
 
 template <typename T, typename OT, int EPI = EPI_FULL>
 __device__ __forceinline__ void epilogue_math32(const GemmParams& p, const uint32_t* acc_bits, long long row,
@@ -167,11 +170,15 @@ __device__ __forceinline__ void epilogue_math32(const GemmParams& p, const uint3
       }
     }
   }
+  if constexpr (EPI == EPI_ROUND) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = to_f32<OT>(from_f32<OT>(v[i]));
+  }
   if (p.residual) {
     float r[32];
     load_row32<OT>(reinterpret_cast<const OT*>(p.residual), p.ldr, row, col, ncols_valid, vec, r);
 #pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = (p.round_first ? to_f32<OT>(from_f32<OT>(v[i])) : v[i]) + r[i];
+    for (int i = 0; i < 32; ++i) v[i] += r[i];
   }
 }
 
@@ -220,7 +227,7 @@ __device__ __forceinline__ void lean_pack32(const GemmParams& p, const uint32_t*
         const uint4 q = *(reinterpret_cast<const uint4*>(rs) + g);
         const T* e = reinterpret_cast<const T*>(&q);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) f[i] = (p.round_first ? to_f32<T>(from_f32<T>(f[i])) : f[i]) + to_f32<T>(e[i]);
+        for (int i = 0; i < 8; ++i) f[i] += to_f32<T>(e[i]);
       }
 #pragma unroll
       for (int i = 0; i < 4; ++i) pk[g * 4 + i] = pack2<T>(f[2 * i], f[2 * i + 1]);
@@ -232,11 +239,11 @@ __device__ __forceinline__ void lean_pack32(const GemmParams& p, const uint32_t*
       float f0 = __uint_as_float(acc_bits[2 * i]) * p.alpha, f1 = __uint_as_float(acc_bits[2 * i + 1]) * p.alpha;
       if (2 * i < ncols_valid) {
         if (b) f0 += to_f32<T>(b[2 * i]);
-        if (rs) f0 = (p.round_first ? to_f32<T>(from_f32<T>(f0)) : f0) + to_f32<T>(rs[2 * i]);
+        if (rs) f0 += to_f32<T>(rs[2 * i]);
       }
       if (2 * i + 1 < ncols_valid) {
         if (b) f1 += to_f32<T>(b[2 * i + 1]);
-        if (rs) f1 = (p.round_first ? to_f32<T>(from_f32<T>(f1)) : f1) + to_f32<T>(rs[2 * i + 1]);
+        if (rs) f1 += to_f32<T>(rs[2 * i + 1]);
       }
       pk[i] = pack2<T>(f0, f1);
     }

@@ -30,7 +30,7 @@ namespace rb {
 
 enum : int { ACT_NONE = 0, ACT_RELU = 1, ACT_GELU = 2, ACT_SILU = 3, ACT_RELU2 = 4 };   // RELU2: the square of relu, forward only
 // Set in the activation argument of rb_gemm and rb_gemm_2cta: the product is rounded to the output's type before the residual is
-// added, as it is when the addition is an operation of its own.
+// added, as it is when the addition is an operation of its own.  (Without a residual the second rounding changes nothing.)
 enum : int { ACT_ROUND_FIRST = 0x100 };
 
 struct GemmParams {
@@ -260,11 +260,15 @@ __device__ __forceinline__ void epilogue_chunk(const GemmParams& p, const uint32
       for (int i = 0; i < 32; ++i) v[i] *= silu_grad(a[i]);
     }
   }
+  if (p.round_first) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = to_f32<OT>(from_f32<OT>(v[i]));
+  }
   if (p.residual) {
     float r[32];
     load_row32<OT>(reinterpret_cast<const OT*>(p.residual), p.ldr, row, col, ncols_valid, vec, r);
 #pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = (p.round_first ? to_f32<OT>(from_f32<OT>(v[i])) : v[i]) + r[i];
+    for (int i = 0; i < 32; ++i) v[i] += r[i];
   }
   store_row32<OT>(reinterpret_cast<OT*>(p.out), p.ldc, row, col, ncols_valid, vec, v);
 }
