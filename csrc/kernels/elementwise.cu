@@ -81,23 +81,24 @@ __global__ void swiglu_fwd_kernel(const T* __restrict__ gu, T* __restrict__ y, l
     y[i] = from_f32<T>(silu_f(g) * u);
   }
 }
-// Sixteen bytes of a row per thread, a row per blockIdx.y: 1555 rows of 11008 took 54 us one number at a time, with a 64-bit division
-// for each, and take 24 (16 us is their way through HBM).
+// Sixteen bytes of a row per thread, the rows' pieces one after the other, so that narrow rows fill their CTAs too (a row per CTA took
+// 37 us for 65536 rows of 16, 6 one number at a time).  1555 rows of 11008: 54 us one number at a time, with a 64-bit division for
+// each, 24 here (16 us is their way through HBM).
 template <typename T>
 __global__ void __launch_bounds__(256)
-    swiglu_fwd_vec_kernel(const T* __restrict__ gu, T* __restrict__ y, long long rows, int F, long long ld) {
+    swiglu_fwd_vec_kernel(const T* __restrict__ gu, T* __restrict__ y, unsigned pieces, unsigned per_row, long long ld) {
   constexpr int VEC = 16 / sizeof(T);
-  const int c = (blockIdx.x * blockDim.x + threadIdx.x) * VEC;
-  if (c >= F) return;
-  for (long long r = blockIdx.y; r < rows; r += gridDim.y) {
-    const uint4 gv = *reinterpret_cast<const uint4*>(gu + r * ld + c), uv = *reinterpret_cast<const uint4*>(gu + r * ld + F + c);
-    const T *g = reinterpret_cast<const T*>(&gv), *u = reinterpret_cast<const T*>(&uv);
-    uint4 ov;
-    T* o = reinterpret_cast<T*>(&ov);
+  const unsigned i = blockIdx.x * 256u + threadIdx.x;
+  if (i >= pieces) return;
+  const unsigned r = i / per_row, c = i - r * per_row;
+  const uint4* row = reinterpret_cast<const uint4*>(gu + r * ld) + c;
+  const uint4 gv = row[0], uv = row[per_row];
+  const T *g = reinterpret_cast<const T*>(&gv), *u = reinterpret_cast<const T*>(&uv);
+  uint4 ov;
+  T* o = reinterpret_cast<T*>(&ov);
 #pragma unroll
-    for (int j = 0; j < VEC; ++j) o[j] = from_f32<T>(silu_f(to_f32<T>(g[j])) * to_f32<T>(u[j]));
-    *reinterpret_cast<uint4*>(y + r * F + c) = ov;
-  }
+  for (int j = 0; j < VEC; ++j) o[j] = from_f32<T>(silu_f(to_f32<T>(g[j])) * to_f32<T>(u[j]));
+  reinterpret_cast<uint4*>(y)[i] = ov;
 }
 // Gated units on gate | up buffers whose output rows are `ldy` apart.  row_gate (may be null, rows ldg apart): every
 // number of a row is multiplied by the sigmoid of row_gate[row].
@@ -421,9 +422,10 @@ int rb_swiglu_fwd(int dtype, const void* gu, void* y, long long rows, int F, lon
   if (rows <= 0) return 0;
   cudaStream_t st = (cudaStream_t)stream;
   const int vec = dtype == rbh::DT_F32 ? 4 : 8;
-  if (F % vec == 0 && ld % vec == 0 && ((reinterpret_cast<uintptr_t>(gu) | reinterpret_cast<uintptr_t>(y)) & 15) == 0) {
-    const dim3 grid((F / vec + 255) / 256, (unsigned)(rows < 65535 ? rows : 65535));
-    RB_DISPATCH_T(dtype, (swiglu_fwd_vec_kernel<T><<<grid, 256, 0, st>>>((const T*)gu, (T*)y, rows, F, ld)));
+  const long long pieces = rows * (F / vec);
+  if (F % vec == 0 && ld % vec == 0 && pieces < (1ll << 31) && ((reinterpret_cast<uintptr_t>(gu) | reinterpret_cast<uintptr_t>(y)) & 15) == 0) {
+    if (pieces == 0) return 0;
+    RB_DISPATCH_T(dtype, (swiglu_fwd_vec_kernel<T><<<(unsigned)((pieces + 255) / 256), 256, 0, st>>>((const T*)gu, (T*)y, (unsigned)pieces, (unsigned)(F / vec), ld)));
     RB_RET_LAST();
   }
   RB_DISPATCH_T(dtype, (swiglu_fwd_kernel<T><<<ew_grid(rows * F, 256), 256, 0, st>>>((const T*)gu, (T*)y, rows, F, ld)));
