@@ -423,8 +423,9 @@ int rb_swiglu_fwd(int dtype, const void* gu, void* y, long long rows, int F, lon
   cudaStream_t st = (cudaStream_t)stream;
   const int vec = dtype == rbh::DT_F32 ? 4 : 8;
   const long long pieces = rows * (F / vec);
-  if (F % vec == 0 && ld % vec == 0 && pieces < (1ll << 31) && ((reinterpret_cast<uintptr_t>(gu) | reinterpret_cast<uintptr_t>(y)) & 15) == 0) {
-    if (pieces == 0) return 0;
+  // Up to 32768 numbers a thread for each: the sixteen bytes of a piece take longer one after the other than a launch does
+  // (16 rows of 8: 1.4 us, 1.7; 16 of 2752 and more: 2.1 against 2.2 and more).
+  if (rows * F > 32768 && F % vec == 0 && ld % vec == 0 && pieces < (1ll << 31) && ((reinterpret_cast<uintptr_t>(gu) | reinterpret_cast<uintptr_t>(y)) & 15) == 0) {
     RB_DISPATCH_T(dtype, (swiglu_fwd_vec_kernel<T><<<(unsigned)((pieces + 255) / 256), 256, 0, st>>>((const T*)gu, (T*)y, (unsigned)pieces, (unsigned)(F / vec), ld)));
     RB_RET_LAST();
   }

@@ -6,8 +6,9 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
-@pytest.mark.parametrize("rows,F,layout", [(1, 8, "plain"), (33, 8, "plain"), (513, 24, "plain"), (7, 2056, "plain"), (5, 12, "plain"),
-                                            (3, 7, "plain"), (40, 16, "pitch"), (9, 64, "offset"), (0, 64, "plain")])
+@pytest.mark.parametrize("rows,F,layout", [(1, 8, "plain"), (33, 8, "plain"), (4097, 8, "plain"), (1366, 24, "plain"), (17, 2056, "plain"),
+                                            (3000, 12, "plain"), (3, 7, "plain"), (5000, 7, "plain"), (2100, 16, "pitch"), (600, 64, "offset"),
+                                            (0, 64, "plain")])
 def test_swiglu(dtype, rows, F, layout):
     from rumus_b200.ops import functional as Fn
     torch.manual_seed(rows + F)
