@@ -680,10 +680,13 @@ int launch_norm_fwd(const void* x, const void* res, const void* gamma, const voi
   norm_fwd_kernel<T, RMS, IT><<<(unsigned)blocks, kNormWarps * 32, 0, st>>>(                       \
       (const T*)x, (const T*)res, (const T*)gamma, (const T*)beta, (T*)y, (T*)h_out, stats, rows, \
       D, eps)
-  // RMS norms of more than four vectors a lane: a CTA per row, as many threads as vectors up to 256.  (Layer norms are met in
-  // training, where there are rows enough for a warp each; another order of their sums would move a step's gradients by rounding.)
+  // RMS norms of more than four vectors a lane: a CTA per row, as many threads as vectors up to 256.  Rows of one vector a thread without a
+  // residual only while they are few: with rows enough for a warp each, a warp per row has fewer barriers and wins (16 bits, D 2048:
+  // 1024 rows 0.66 of its time, 2048 0.93, 3000 1.11, 8192 1.21, 40000 1.14; 32 bits, D 1024: 1024 rows 0.90, 2048 1.10).  With a residual, or
+  // more vectors a thread, a CTA per row is ahead at every count (0.5 to 1.0).  (Layer norms are met in training, where there are
+  // rows enough for a warp each; another order of their sums would move a step's gradients by rounding.)
   const int vecs = D / VEC;
-  if (RMS && vec && iters > 4 && vecs <= 4 * 256 && rows < (1ll << 31)) {
+  if (RMS && vec && iters > 4 && vecs <= 4 * 256 && (vecs > 256 || res || rows <= 256 * VEC) && rows < (1ll << 31)) {
     const int per = (vecs + 255) / 256;
     const int threads = ((vecs + per - 1) / per + 31) / 32 * 32;
 #define RB_NORM_WIDE(V)                                                                           \

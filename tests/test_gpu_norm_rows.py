@@ -19,3 +19,15 @@ def test_rms_norm_wide_rows(dtype, D):
         ref = v.double() * torch.rsqrt(v.double().pow(2).mean(-1, keepdim=True) + 1e-6) * w.double()
         # one rounding of the result, and of the sum and root in 32 bits
         assert ((got.double() - ref).norm() / ref.norm()).item() < {torch.bfloat16: 2 ** -8, torch.float16: 2 ** -11}.get(dtype, 1e-6)
+
+
+# rows of one vector a thread: a CTA each up to 2048 (1024 in 32 bits), a warp each beyond
+@pytest.mark.parametrize("dtype,D", [(torch.bfloat16, 1288), (torch.float16, 2048), (torch.float32, 1024)])
+@pytest.mark.parametrize("rows", [1, 1024, 1025, 2048, 2049, 3001])
+def test_rms_norm_many_rows(dtype, D, rows):
+    from rumus_b200.ops import functional as F
+    torch.manual_seed(rows)
+    x, w = torch.randn(rows, D, device="cuda").to(dtype), torch.randn(D, device="cuda").to(dtype)
+    y = F.rms_norm(x, w, 1e-6)
+    ref = x.double() * torch.rsqrt(x.double().pow(2).mean(-1, keepdim=True) + 1e-6) * w.double()
+    assert ((y.double() - ref).norm() / ref.norm()).item() < {torch.bfloat16: 2 ** -8, torch.float16: 2 ** -11}.get(dtype, 1e-6)
