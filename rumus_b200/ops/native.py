@@ -172,6 +172,15 @@ def _use_2cta(M: int, N: int) -> bool:
     return ((M + 255) // 256) * ((N + 255) // 256) * 4 >= sm_count()
 
 
+def _few_rows_fit(M: int, N: int, K: int) -> bool:
+    """33 to 64 rows: whether the few-rows kernel is ahead of 128-row tiles.  Below 8192 columns always; beyond, while the clusters of
+    four CTAs that share K are all resident at once (71 of them, 9088 columns, on 148 SMs) and there is K enough for what
+    adding up a cluster's sums of more than 48 rows takes.  Of the other kernel's time: N 8192 to 9088 0.78 to 0.92 (33 rows), 0.85 to 1.0
+    (64 rows, K 1024 and more), 1.05 to 1.12 (64 rows, K 512); N 9216, a second wave, 1.1 to 1.3 (33 rows), 1.2 to 1.7 (64)."""
+    tiles = (N + 127) // 128
+    return N < 8192 or (25 * tiles <= 12 * sm_count() and (M <= 48 or K >= 1024))
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, *, bias: Optional[torch.Tensor] = None,
          act: Optional[str] = None, residual: Optional[torch.Tensor] = None,
          aux_out: bool = False, aux_in: Optional[torch.Tensor] = None, dact: Optional[str] = None,
@@ -235,9 +244,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, bias: Optional[torch.Tensor] = Non
         assert aux_in.dtype == odt and aux_in.shape == (M, N) and aux_in.stride(1) == 1
     act_code = ACT_CODES[act] | (0x100 if round_first else 0)
     few = M <= 128 and not round_first and not at and bt and a.dtype == torch.bfloat16 and not aux_out and aux_in is None and dact is None
-    # more than 32 rows: only where 128-row tiles of the weight leave half of the SMs idle, so that four CTAs or more share K
-    # (64 rows, K 2048: N 8192 12.8 us, 13.9 on the other kernel; N 11264, two CTAs, 18.2 and 15.1)
-    if path == 4 or (path == 0 and few and (M <= 32 or (M <= 64 and 2 * ((N + 127) // 128) <= sm_count())) and N * K >= 1 << 16 and split_k == 0 and bn == 0
+    if path == 4 or (path == 0 and few and (M <= 32 or (M <= 64 and _few_rows_fit(M, N, K))) and N * K >= 1 << 16 and split_k == 0 and bn == 0
                      and max_ctas == 0):
         rc = 13 if not few else L.rb_gemm_rows(
             dt, ptr(a), lda, ptr(b), ldb, M, N, K, ptr(out), out.stride(0) if M > 1 else N, out_f32, ptr(bias), ptr(residual),

@@ -49,3 +49,15 @@ def test_sums_do_not_depend_on_the_other_rows():
     whole = native.gemm(a, w.t(), out_dtype=F32)
     for i in (0, 7, 15):
         assert torch.equal(native.gemm(a[i:i + 1], w.t(), out_dtype=F32)[0], whole[i])
+
+
+# the edges of the rule for 33 to 64 rows: a wave of clusters, K for their sums
+@pytest.mark.parametrize("M,N,K,path", [(33, 8100, 512, 4), (48, 9088, 512, 4), (49, 9088, 512, 1), (64, 9088, 1024, 4), (33, 9089, 512, 1),
+                                         (64, 8191, 512, 4), (65, 1024, 512, 1)])
+def test_more_than_32_rows(M, N, K, path):
+    from rumus_b200.ops import native
+    torch.manual_seed(M + N)
+    a, w = torch.randn(M, K, device="cuda").to(BF), torch.randn(N, K, device="cuda").to(BF)
+    got = native.gemm(a, w.t())
+    assert native.gemm.last_path == path
+    assert _rel(got, (a.double() @ w.double().T).cpu()) < 3e-3
