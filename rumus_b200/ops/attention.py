@@ -32,7 +32,18 @@ def _tma_ok(t: torch.Tensor) -> bool:
             and all((t.stride(i) * t.element_size()) % 16 == 0 for i in range(3)))
 
 
-F32_MAX_ROWS = 1024
+def f32_max_rows(Sq: int, Sk: int, D: int, causal: bool) -> int:
+    """Queries and keys up to which the 32-bit kernels are ahead of the batched products they replace.  A row's keys are a serial chain,
+    which the products' tiles are not, and a key read from shared memory serves 128 / (D / 16) rows, so long rows, wide heads and rows
+    without a mask are where the products catch up.  Forward and backward, of the products' time, 1 to 64 x 8 batches and heads:
+    causal 0.16 to 0.83 up to 1024 keys; not causal, heads of 32 0.16 to 0.80 up to 1024, of 64 0.2 to 1.0 up to 768 and 1.05 at 1024, of
+    128 0.3 to 1.0 up to 192 and 1.05 to 1.27 from 256; other numbers of keys than of queries 0.3 to 0.95 up to 384 (192 for
+    heads of 128), 1.1 to 1.2 for 16 or 64 queries of 512 keys and more."""
+    if Sq == Sk and (causal or D <= 32):
+        return 1024
+    if D <= 64:
+        return 768 if Sq == Sk else 384
+    return 192
 
 
 def f32_covers(q, k, v, causal: bool) -> bool:
@@ -41,14 +52,14 @@ def f32_covers(q, k, v, causal: bool) -> bool:
     if len(q) != 4 or len(k) != 4 or k != v:
         return False
     (B, Sq, H, D), Sk = q, k[1]
-    return k == (B, Sk, H, D) and D in (16, 32, 64, 128) and 0 < Sk <= F32_MAX_ROWS and 0 < Sq and (Sk >= Sq or not causal)
+    return k == (B, Sk, H, D) and D in (16, 32, 64, 128) and 0 < Sk and 0 < Sq and (Sk >= Sq or not causal)
 
 
 def f32_covered(q, k, v, causal: bool) -> bool:
-    """Whether the 32-bit kernels take these tensors.  All others, sequences beyond ``F32_MAX_ROWS`` among them, stay with the batched
-    products."""
+    """Whether the 32-bit kernels take these tensors; all others stay with the batched products."""
     return (q.is_cuda and q.dtype == k.dtype == v.dtype == torch.float32 and q.device == k.device == v.device
-            and f32_covers(tuple(q.shape), tuple(k.shape), tuple(v.shape), causal))
+            and f32_covers(tuple(q.shape), tuple(k.shape), tuple(v.shape), causal)
+            and max(q.shape[1], k.shape[1]) <= f32_max_rows(q.shape[1], k.shape[1], q.shape[3], causal))
 
 
 def attn_f32_forward(q, k, v, causal: bool, scale: float):

@@ -54,3 +54,12 @@ def test_16_bit_forward_turns_other_shapes_away(q, k, v, types):
     dt = {"b": torch.bfloat16, "h": torch.float16}
     with pytest.raises(ValueError):
         fa_forward(*(torch.zeros(s, dtype=dt[t]) for s, t in zip((q, k, v), types)), True, 0.1)
+
+
+@pytest.mark.parametrize("Sq,Sk,D,causal,rows", [
+    (1024, 1024, 128, True, 1024), (1024, 1024, 32, False, 1024), (1024, 1024, 64, False, 768), (256, 256, 128, False, 192),
+    (16, 512, 64, True, 384), (16, 512, 16, False, 384), (64, 256, 128, True, 192),
+])
+def test_32_bit_rows_go_to_the_quicker_kernels(Sq, Sk, D, causal, rows):
+    from rumus_b200.ops.attention import f32_max_rows
+    assert f32_max_rows(Sq, Sk, D, causal) == rows
