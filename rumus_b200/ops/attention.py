@@ -48,11 +48,13 @@ def f32_max_rows(Sq: int, Sk: int, D: int, causal: bool) -> int:
 
 def f32_covers(q, k, v, causal: bool) -> bool:
     """Whether heads of these shapes are what the 32-bit kernels (``csrc/kernels/attn_f32.cu``) read and write: the batch, the
-    heads and their size of k and v are q's (the kernels step through all three by q's sizes), a key for every row."""
+    heads and their size of k and v are q's (the kernels step through all three by q's sizes), a key for every row, and no more
+    batches and heads than a grid's third and second dimension hold."""
     if len(q) != 4 or len(k) != 4 or k != v:
         return False
     (B, Sq, H, D), Sk = q, k[1]
-    return k == (B, Sk, H, D) and D in (16, 32, 64, 128) and 0 < Sk and 0 < Sq and (Sk >= Sq or not causal)
+    return (k == (B, Sk, H, D) and D in (16, 32, 64, 128) and 0 < Sk and 0 < Sq and (Sk >= Sq or not causal)
+            and B <= 65535 and H <= 65535)
 
 
 def f32_covered(q, k, v, causal: bool) -> bool:

@@ -17,6 +17,9 @@ import torch
     ((4, 8, 2, 32), (4, 7, 2, 32), (4, 7, 2, 32), True, False),        # a row without keys
     ((4, 8, 2, 32), (4, 7, 2, 32), (4, 7, 2, 32), False, True),
     ((8, 2, 32), (8, 2, 32), (8, 2, 32), True, False),
+    ((65535, 2, 2, 16), (65535, 2, 2, 16), (65535, 2, 2, 16), True, True),
+    ((65536, 2, 2, 16), (65536, 2, 2, 16), (65536, 2, 2, 16), True, False),
+    ((1, 2, 65536, 16), (1, 2, 65536, 16), (1, 2, 65536, 16), True, False),
 ])
 def test_32_bit_heads(q, k, v, causal, covered):
     from rumus_b200.ops.attention import f32_covers
