@@ -105,7 +105,8 @@ __global__ void __launch_bounds__(AF_THREADS) attn_f32_fwd_kernel(const AttnF32P
         if (j0 + j + u >= keys) s[u] = -INFINITY;
       }
       const float mn = fmaxf(m, fmaxf(fmaxf(s[0], s[1]), fmaxf(s[2], s[3])));
-      if (mn != -INFINITY) {
+      // no key of the group is seen by this row: all of them are -inf.  fmaxf passes over NaN, a sum does not.
+      if (mn != -INFINITY || (s[0] + s[1]) + (s[2] + s[3]) != -INFINITY) {
         const float f = expf(m - mn);
         l *= f;
 #pragma unroll

@@ -70,3 +70,24 @@ def test_packed_rows_of_other_layouts(layout):
         out += [o, torch.autograd.grad(o, t, g)[0]]
     for a, b in zip(got, want):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("D", [16, 128])
+def test_numbers_that_are_none(D, causal):
+    """NaN and infinite scores reach the result where a softmax in 64 bits has them, also as the first keys of a row."""
+    from rumus_b200.ops.attention import attention_f32
+    torch.manual_seed(D)
+    q, k, v = (torch.randn(2, 40, 2, D, device="cuda") for _ in range(3))
+    k[0, :4, 0] = float("nan")              # one group of keys, the first
+    k[0, 9, 1, 0] = float("inf")            # scores of +inf and -inf
+    k[1, 33, 0, 1] = float("nan")
+    v[1, 2, 1, 3] = float("inf")
+    o = attention_f32(q, k, v, causal)
+    ref = _ref(q.double(), k.double(), v.double(), causal, D ** -0.5)
+    some = torch.isfinite(ref)
+    assert torch.equal(torch.isnan(o[0, :, 0]), torch.isnan(ref[0, :, 0])) and torch.isnan(o[0, :, 0]).all()
+    assert torch.equal(torch.isfinite(o)[0], some[0]) and torch.equal(torch.isfinite(o)[1, :, 0], some[1, :, 0])
+    seen = torch.arange(40, device="cuda") >= 2 if causal else torch.ones(40, dtype=torch.bool, device="cuda")
+    assert torch.isinf(o[1, seen, 1, 3]).all()
+    assert ((o - ref)[some & torch.isfinite(o)].norm() / ref[some].norm()).item() < 1e-5
