@@ -244,27 +244,23 @@ __global__ void __launch_bounds__(320, 1)
       tmem_ld_wait();
       const bool need_mask = (kv0 + C::BN > p.Sk) || (p.causal && kv0 + C::BN - 1 > q0 + off);
       const int last = (p.causal ? min(p.Sk - 1, row + off) : p.Sk - 1) - kv0;       // last column that counts
-      if (need_mask) {
+      if (need_mask) {                           // what is masked ends as exp2(-inf) below
 #pragma unroll
         for (int c = 0; c < 4; ++c)
 #pragma unroll
           for (int i = 0; i < 32; ++i)
-            if (c * 32 + i > last) s[c][i] = 0xff800000u;
+            if (c * 32 + i > last) s[c][i] = NEGATIVE ? 0x7f800000u : 0xff800000u;
       }
-      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+      // the largest score: of the largest S, with a negative scale of the smallest (of a row that sees no key of this tile: -inf)
+      auto further = [](float a, float b) { return NEGATIVE ? fminf(a, b) : fmaxf(a, b); };
+      constexpr float NONE = NEGATIVE ? INFINITY : -INFINITY;
+      float mx4[4] = {NONE, NONE, NONE, NONE};
 #pragma unroll
       for (int c = 0; c < 4; ++c)
 #pragma unroll
         for (int i = 0; i < 32; i += 2)
-          mx4[(i >> 1) & 3] = fmaxf(fmaxf(mx4[(i >> 1) & 3], __uint_as_float(s[c][i])), __uint_as_float(s[c][i + 1]));
-      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-      if (NEGATIVE && need_mask) {               // what is masked has to end as exp2(-inf) below
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-#pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (c * 32 + i > last) s[c][i] = 0x7f800000u;
-      }
+          mx4[(i >> 1) & 3] = further(further(mx4[(i >> 1) & 3], __uint_as_float(s[c][i])), __uint_as_float(s[c][i + 1]));
+      const float mx = further(further(mx4[0], mx4[1]), further(mx4[2], mx4[3]));
       const float m_new = fmaxf(m_used, mx * p.scale_log2);
       const bool need = m_new > m_used + 8.0f;  // also true on this warpgroup's first tile (m_used = -inf)
       if (__any_sync(0xffffffffu, need)) {       // the TMEM accesses below are warp-wide: uniform branch

@@ -28,3 +28,27 @@ def test_flash_forward_edges(D, Sq, Sk, H, Hkv, causal, scale):
     seen = torch.isfinite(want)
     assert torch.equal(torch.isfinite(lse), seen) and (lse.double() - want)[seen].abs().max() < 1e-4
     assert native.read_status() == 0
+
+
+# rows that see no key of a tile (Sk - Sq no multiple of 128), and scores that range beyond what 16 bits hold of exp2
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("Sq,Sk,causal,scale", [(100, 300, True, -0.1), (130, 257, True, -0.1), (300, 130, True, -0.1), (1, 129, True, -0.1),
+                                                 (200, 384, False, -2.0), (260, 384, True, -2.0), (260, 384, True, 2.0), (100, 300, True, 2.0)])
+def test_flash_forward_negative_scales(D, dtype, Sq, Sk, causal, scale):
+    from rumus_b200.ops import native
+    from rumus_b200.ops.attention import fa_forward
+    torch.manual_seed(Sq + Sk)
+    q, k, v = (torch.randn(2, S, 2, D, device="cuda").to(dtype) for S in (Sq, Sk, Sk))
+    o, lse, _ = fa_forward(q, k, v, causal, scale)
+    s = torch.einsum("bihd,bjhd->bhij", q.double(), k.double()) * scale
+    if causal:
+        s = s.masked_fill(~torch.ones(Sq, Sk, dtype=torch.bool, device="cuda").tril(Sk - Sq), float("-inf"))
+    ref = torch.einsum("bhij,bjhd->bihd", s.softmax(-1).nan_to_num(0.0), v.double())
+    # weights and results rounded to 8 (11) bits; the scores' own rounding, 2^-24 of up to 2 * 128 each way, is below that
+    assert torch.isfinite(o).all() and ((o.double() - ref).norm() / ref.norm()).item() < 2 ** -8
+    want = torch.logsumexp(s, -1)
+    seen = torch.isfinite(want)
+    assert torch.equal(torch.isfinite(lse), seen) and not torch.isnan(lse).any()
+    assert (lse.double() - want)[seen].abs().max() < 1e-4 * max(1.0, want[seen].abs().max().item() / 10)
+    assert native.read_status() == 0
