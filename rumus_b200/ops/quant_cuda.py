@@ -31,9 +31,9 @@ native.register_signature("rb_q8_dequantize", [I, P, P, I, I, I, P])
 ROWS_MAX_M = 48            # rows of the register-fed tensor-core kernel; above, a dense copy is quicker (64 rows, the four
                            # products of a 7B layer: 233 us by that kernel with eight groups of rows, 201 us)
 GEMV_MAX_M = 32            # rows one GEMV launch handles (accumulators in registers)
-GEMV_CHUNKED_MAX_M = 8     # batches up to this size use the GEMV; larger ones dequantise + tcgen05 GEMM
-                           # (measured crossover on K 4096 x N 12288: GEMV 81 us at 8 rows, 118 us at 16;
-                           # dequantise + GEMM 85-97 us for any batch up to 128)
+GEMV_CHUNKED_MAX_M = 8     # of what the rows kernel does not take, batches up to this size use the GEMV; larger ones expand the weight
+                           # (K 4096 x N 12288, before that kernel: GEMV 81 us at 8 rows, 118 us at 16; dequantise + GEMM
+                           # 85-97 us for any batch up to 128)
 
 
 def int4_dequant(qw, dtype: torch.dtype) -> torch.Tensor:
@@ -45,9 +45,9 @@ def int4_dequant(qw, dtype: torch.dtype) -> torch.Tensor:
     return dense
 
 
-# Batches of GEMV_CHUNKED_MAX_M+1 .. W4A16_MAX_M rows take the fused W4A16 tcgen05 kernel
-# (csrc/kernels/w4a16_gemm.cu), which expands the packed weight inside shared memory instead of
-# writing a dense 16-bit copy (RB_W4A16=0 switches back to dequantise + GEMM).
+# Batches of GEMV_CHUNKED_MAX_M + 1 .. W4A16_ROUTE_MAX_M rows expand the packed weight inside the kernel that multiplies it, in registers
+# (ROWS_MAX_M, groups that are multiples of 128) or in shared memory (csrc/kernels/w4a16_gemm.cu, other groups), instead of
+# writing a dense 16-bit copy.  RB_W4A16=0 switches both back to dequantise + GEMM: each weight is then rounded once, from 32 bits.
 W4A16_MAX_M = 128
 W4A16_ROUTE_MAX_M = 48     # above this the split-K additions of the fused kernel cost more than a dense copy
 
@@ -149,7 +149,7 @@ def int4_matmul(x: torch.Tensor, qw, bias=None, out=None, residual=None) -> torc
     if residual is not None:
         assert residual.shape == (M, qw.n) and residual.dtype == x.dtype
         residual = residual.contiguous()
-    if bias is None or bias.dtype == x.dtype:
+    if (bias is None or bias.dtype == x.dtype) and (M <= GEMV_CHUNKED_MAX_M or w4a16_enabled()):
         y = int4_matmul_rows(x, qw, bias, out, residual)
         if y is not None:
             return y

@@ -66,3 +66,15 @@ def test_int4_rows_infinite_activations():
     y = Q.int4_matmul_rows(x, q)
     assert torch.equal(torch.isnan(y), torch.isnan(ref)) and torch.equal(y[torch.isinf(ref)], ref[torch.isinf(ref)])
     assert _rel(y[[0, 2]], ref[[0, 2]].double()) < 2 ** -8
+
+
+@pytest.mark.parametrize("M,dense", [(8, False), (9, True), (48, True)])
+def test_int4_dense_weights_on_request(M, dense, monkeypatch):
+    """RB_W4A16=0: more than eight rows are multiplied with the weights of a dense copy, rounded once."""
+    from rumus_b200.ops import native, quant_cuda as Q
+    monkeypatch.setenv("RB_W4A16", "0")
+    x, q = _case(M, 1024, 264, torch.bfloat16, torch.float32, M)
+    res = torch.randn(M, 264, device="cuda").bfloat16()
+    want = native.gemm(x, Q.int4_dequant(q, x.dtype))
+    assert torch.equal(Q.int4_matmul(x, q), want) is dense
+    assert _rel(Q.int4_matmul(x, q, residual=res), want.double() + res.double()) < 2 ** -7
