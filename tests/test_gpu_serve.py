@@ -36,6 +36,10 @@ def test_int4_gemv_all_row_buckets(M, monkeypatch):
     from rumus_b200.nn.quant import QuantizedTensor
     from rumus_b200.ops import quant_cuda as Q
     monkeypatch.setattr(Q, "GEMV_CHUNKED_MAX_M", 128)
+    monkeypatch.setattr(Q, "ROWS_MAX_M", 0)              # the kernel that is asked first
+    calls = []
+    gemv = Q.native.lib().rb_int4_gemv
+    monkeypatch.setattr(Q.native.lib(), "rb_int4_gemv", lambda *a: calls.append(a) or gemv(*a))
     torch.manual_seed(M)
     K, N = 1160, 520     # K is not a multiple of the group size, N not of 512
     w = torch.randn(K, N) * 0.05
@@ -45,6 +49,7 @@ def test_int4_gemv_all_row_buckets(M, monkeypatch):
     y = Q.int4_matmul(x, q, bias)
     ref = x.float() @ q.dequantize(torch.float32) + bias.float()
     assert _rel(y, ref) < 1e-2
+    assert len(calls) == (M + Q.GEMV_MAX_M - 1) // Q.GEMV_MAX_M
 
 
 def test_q8_roundtrip_and_matmul():
