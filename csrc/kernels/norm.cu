@@ -138,26 +138,24 @@ __global__ void __launch_bounds__(kNormWarps * 32)
   }
 }
 
-// A CTA per row, VPT vectors a thread: wide rows.  With a warp per row a lane works through up to 32 vectors one after the
+// RMS norms, a CTA per row, VPT vectors a thread: wide rows.  With a warp per row a lane works through up to 32 vectors one after the
 // other and one row keeps one warp busy; here the whole row is one round of loads, which is what counts both for a few rows (decode) and,
 // as more loads are in flight per SM, for many.  RMS norm of 1 to 1555 rows of 4096: 10.7 us with a warp per row, 2.4 to 6.4.
-template <typename T, bool RMS, int VPT>
+template <typename T, int VPT>
 __global__ void __launch_bounds__(256)
-    norm_fwd_wide_kernel(const T* __restrict__ x, const T* __restrict__ res, const T* __restrict__ gamma,
-                         const T* __restrict__ beta, T* __restrict__ y, T* __restrict__ h_out,
-                         float* __restrict__ stats, int D, float eps) {
+    rms_norm_fwd_wide_kernel(const T* __restrict__ x, const T* __restrict__ res, const T* __restrict__ gamma, T* __restrict__ y,
+                             T* __restrict__ h_out, float* __restrict__ stats, int D, float eps) {
   constexpr int VEC = Vec16<T>::N;
-  __shared__ float s_red[2][8];
+  __shared__ float s_red[8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   const long long base = (long long)blockIdx.x * D;
-  Vec16<T> v[VPT], g[VPT], b[VPT];
+  Vec16<T> v[VPT], g[VPT];
 #pragma unroll
   for (int i = 0; i < VPT; ++i) {
     const int c = (i * blockDim.x + threadIdx.x) * VEC;
     if (c < D) {
       v[i].raw = *reinterpret_cast<const uint4*>(x + base + c);
       g[i].raw = *reinterpret_cast<const uint4*>(gamma + c);
-      if (!RMS && beta) b[i].raw = *reinterpret_cast<const uint4*>(beta + c);
       if (res) {
         Vec16<T> r;
         r.raw = *reinterpret_cast<const uint4*>(res + base + c);
@@ -167,38 +165,21 @@ __global__ void __launch_bounds__(256)
       }
     }
   }
-  auto total = [&](float a, int k) {
-    a = warp_sum(a);
-    if (lane == 0) s_red[k][warp] = a;
-    __syncthreads();
-    float r = 0.f;
-    for (int w = 0; w < nwarps; ++w) r += s_red[k][w];
-    return r;
-  };
-  float mean = 0.f;
-  if (!RMS) {
-    float sum = 0.f;
-#pragma unroll
-    for (int i = 0; i < VPT; ++i)
-      if ((i * blockDim.x + threadIdx.x) * VEC < D) {
-#pragma unroll
-        for (int j = 0; j < VEC; ++j) sum += v[i].get(j);
-      }
-    mean = total(sum, 0) / D;
-  }
   float sumsq = 0.f;
 #pragma unroll
   for (int i = 0; i < VPT; ++i)
     if ((i * blockDim.x + threadIdx.x) * VEC < D) {
 #pragma unroll
-      for (int j = 0; j < VEC; ++j) {
-        const float d = v[i].get(j) - mean;
-        sumsq += d * d;
-      }
+      for (int j = 0; j < VEC; ++j) sumsq += v[i].get(j) * v[i].get(j);
     }
-  const float rstd = rsqrtf(total(sumsq, 1) / D + eps);
+  sumsq = warp_sum(sumsq);
+  if (lane == 0) s_red[warp] = sumsq;
+  __syncthreads();
+  float total = 0.f;
+  for (int w = 0; w < nwarps; ++w) total += s_red[w];
+  const float rstd = rsqrtf(total / D + eps);
   if (threadIdx.x == 0 && stats) {
-    stats[(long long)blockIdx.x * 2] = mean;
+    stats[(long long)blockIdx.x * 2] = 0.f;
     stats[(long long)blockIdx.x * 2 + 1] = rstd;
   }
 #pragma unroll
@@ -207,11 +188,7 @@ __global__ void __launch_bounds__(256)
     if (c < D) {
       Vec16<T> o;
 #pragma unroll
-      for (int j = 0; j < VEC; ++j) {
-        float f = (v[i].get(j) - mean) * rstd * g[i].get(j);
-        if (!RMS && beta) f += b[i].get(j);
-        o.set(j, f);
-      }
+      for (int j = 0; j < VEC; ++j) o.set(j, v[i].get(j) * rstd * g[i].get(j));
       *reinterpret_cast<uint4*>(y + base + c) = o.raw;
     }
   }
@@ -685,19 +662,21 @@ int launch_norm_fwd(const void* x, const void* res, const void* gamma, const voi
   // 1024 rows 0.66 of its time, 2048 0.93, 3000 1.11, 8192 1.21, 40000 1.14; 32 bits, D 1024: 1024 rows 0.90, 2048 1.10).  With a residual, or
   // more vectors a thread, a CTA per row is ahead at every count (0.5 to 1.0).  (Layer norms are met in training, where there are
   // rows enough for a warp each; another order of their sums would move a step's gradients by rounding.)
-  const int vecs = D / VEC;
-  if (RMS && vec && iters > 4 && vecs <= 4 * 256 && (vecs > 256 || res || rows <= 256 * VEC) && rows < (1ll << 31)) {
-    const int per = (vecs + 255) / 256;
-    const int threads = ((vecs + per - 1) / per + 31) / 32 * 32;
-#define RB_NORM_WIDE(V)                                                                           \
-  norm_fwd_wide_kernel<T, RMS, V><<<(unsigned)rows, threads, 0, st>>>(                            \
-      (const T*)x, (const T*)res, (const T*)gamma, (const T*)beta, (T*)y, (T*)h_out, stats, D, eps)
-    if (per == 1) RB_NORM_WIDE(1);
-    else if (per == 2) RB_NORM_WIDE(2);
-    else RB_NORM_WIDE(4);
+  if constexpr (RMS) {
+    const int vecs = D / VEC;
+    if (vec && iters > 4 && vecs <= 4 * 256 && (vecs > 256 || res || rows <= 256 * VEC) && rows < (1ll << 31)) {
+      const int per = (vecs + 255) / 256;
+      const int threads = ((vecs + per - 1) / per + 31) / 32 * 32;
+#define RB_NORM_WIDE(V)                                                   \
+  rms_norm_fwd_wide_kernel<T, V><<<(unsigned)rows, threads, 0, st>>>(     \
+      (const T*)x, (const T*)res, (const T*)gamma, (T*)y, (T*)h_out, stats, D, eps)
+      if (per == 1) RB_NORM_WIDE(1);
+      else if (per == 2) RB_NORM_WIDE(2);
+      else RB_NORM_WIDE(4);
 #undef RB_NORM_WIDE
-    cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? 0 : 3000 + (int)e;
+      cudaError_t e = cudaGetLastError();
+      return e == cudaSuccess ? 0 : 3000 + (int)e;
+    }
   }
   if (!vec || iters > 32) RB_NORM_LAUNCH(0);
   else if (iters <= 1) RB_NORM_LAUNCH(1);
