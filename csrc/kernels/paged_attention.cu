@@ -5,8 +5,8 @@
 // (rumus-serve/src/model.rs:14-142) and scans the vocabulary on the CPU for the argmax
 // (rumus-serve/src/scheduler.rs:101-135); none of these kernels has a counterpart there.
 //
-// Cache layout: k_cache / v_cache [num_blocks, block_size, Hkv, D] (token-major) or, in the `_hm`
-// entry points, [num_blocks, Hkv, block_size, D] (head-major); a sequence's logical token t lives in
+// Cache layout: k_cache / v_cache [num_blocks, block_size, Hkv, D] (token-major) or, with `head_major` and in
+// rb_kv_append_hm, [num_blocks, Hkv, block_size, D] (head-major); a sequence's logical token t lives in
 // physical block block_table[b][t / block_size] at offset t % block_size.
 #include "warp_mma.cuh"
 
@@ -339,8 +339,8 @@ __global__ void __launch_bounds__(256)
 
 extern "C" {
 
-// CTAs that share the keys of one (row, head): parts of at most 512 tokens, shorter ones (down to 64 tokens) while the rows and
-// heads alone leave less than four CTAs to an SM.
+// CTAs that share the keys of one (row, head): parts of at most 512 tokens up to 8192 tokens (sixteen parts, longer ones beyond), shorter
+// ones (down to 64 tokens) while the rows and heads alone leave less than four CTAs to an SM.
 int rb_paged_decode_splits(int max_ctx, int rows_heads) {
   const int fill = (4 * rbh::sm_count() + rows_heads - 1) / (rows_heads > 0 ? rows_heads : 1);
   int s = fill < (max_ctx + 63) / 64 ? fill : (max_ctx + 63) / 64;
