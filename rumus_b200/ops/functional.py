@@ -656,9 +656,9 @@ def sdpa_reference(q, k, v, causal: bool, scale: Optional[float] = None):
 
 def flash_attention_packed(qkv, heads: int, kv_heads: int, causal: bool = True,
                            scale: Optional[float] = None):
-    """Attention over the fused projection output ``[B, S, (heads + 2*kv_heads) * 128]`` (CUDA,
-    16-bit): same result as splitting and calling ``flash_attention``, without the gradient
-    concatenation."""
+    """Attention over the fused projection output ``[B, S, (heads + 2*kv_heads) * head_dim]`` on a GPU, 16-bit with heads of 128 or
+    32-bit with as many key heads as query heads, of 16, 32, 64 or 128: same result as splitting and calling
+    ``flash_attention``, without the gradient concatenation."""
     from .attention import flash_attention_packed as _packed
     return _packed(qkv, heads, kv_heads, causal, scale)
 

@@ -1,8 +1,9 @@
 """Llama with INT4 (AWQ-layout) weights for the serving engine: weights, paged attention and the decoder stack.
 
 Weights are INT4 group-128 with fp16 scales, sharded Megatron-style across the tensor-parallel group (qkv /
-gate-up by output columns, out-proj / down by input rows on group boundaries); decode uses the streaming GEMV
-or the fused W4A16 kernel, prefill the dequant + tcgen05 GEMM path.
+gate-up by output columns, out-proj / down by input rows on group boundaries); decode batches of up to 48 rows feed
+the four-bit weights to the tensor cores from registers (``csrc/kernels/int4_rows.cu``), prefill expands them to a
+dense copy for the tcgen05 GEMM.
 """
 from __future__ import annotations
 
