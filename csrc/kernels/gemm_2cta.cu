@@ -90,7 +90,7 @@ int launch_gemm_2cta_flavour(GemmArgs& a, int mt) {
 // back under the power cap (bf16, M 16384): wide outputs (N 8192: 1241 vs 1220 TFLOP/s, N 50304: 1218
 // vs 1181) gain from the larger tile, narrow ones (N 2048: 1273 vs 1300 at K 8192, 1078 vs 1143 at
 // K 2048) do not; neither does a problem whose 512-row tiles leave the last wave of clusters emptier or more of their rows
-// beyond M (1555 rows, the four products of a 7B layer: 582 us with 512-row tiles, 537 with 256).
+// beyond M (1555 rows, K 4096: N 12288 144 us with 512-row tiles, 129 with 256, N 22016 245 and 229).
 int pick_pair_mt(int M, int N, int clusters) {
   if (M <= 256 || N < 4096) return 1;
   auto waves = [&](int bm) {
